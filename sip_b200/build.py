@@ -87,7 +87,9 @@ def build(clean: bool = False, verbose: bool = False, jobs: int | None = None) -
         if _stale(obj, src):
             todo.append((src, obj))
     # device-heavy translation units first, so that the longest compiles start at once
-    todo.sort(key=lambda so: (not so[0].endswith(".cu"), -os.path.getsize(so[0]) if "row_inst_32" not in so[0] else -1e9))
+    slow = ("row_inst_32", "pair_tile_fwd", "pair_tile_inv", "pair_batch")
+    todo.sort(key=lambda so: (not so[0].endswith(".cu"),
+                              -1e9 if any(k in so[0] for k in slow) else -os.path.getsize(so[0])))
     if todo:
         with cf.ThreadPoolExecutor(max_workers=jobs or min(8, os.cpu_count() or 4)) as ex:
             for src, warn in ex.map(lambda so: _compile(so[0], so[1], verbose), todo):

@@ -113,5 +113,12 @@ __device__ __forceinline__ void st_stream(float2 *p, float2 v)
 {
     asm volatile("st.global.L1::no_allocate.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
 }
+// two adjacent elements, p 16-byte aligned
+__device__ __forceinline__ void st_stream(float2 *p, float2 v, float2 w)
+{
+    asm volatile("st.global.L1::no_allocate.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(w.x),
+                 "f"(w.y)
+                 : "memory");
+}
 
 }  // namespace sipfft

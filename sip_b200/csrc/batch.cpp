@@ -224,9 +224,13 @@ struct BatchPlan {
     bool forward = true;
     std::vector<int64_t> sizes, batches;
     std::vector<BatchSeg> segs;
+    bool pairs = false;  // every segment is a pair tile (two transforms per thread): pair_segs instead of segs
+    std::vector<PairSeg> pair_segs;
     std::vector<int2> items;
     std::vector<std::string> seg_what;
     BatchSeg *d_segs = nullptr;
+    PairSeg *d_pair_segs = nullptr;
+    int buf_words = 0;  // tile buffer of the pair kernel
     int2 *d_items = nullptr;
     int *d_counters = nullptr;  // [0] = item counter, [1 + s] = tiles done of segment s
     size_t ws_bytes = 0;
@@ -248,6 +252,7 @@ struct BatchPlan {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
         cudaFree(d_segs);
+        cudaFree(d_pair_segs);
         cudaFree(d_items);
         cudaFree(d_counters);
         cudaGetLastError();
@@ -259,6 +264,8 @@ namespace {
 std::string build_batch_with(BatchPlan &bp)
 {
     bp.segs.clear();
+    bp.pair_segs.clear();
+    bp.buf_words = 0;
     bp.items.clear();
     bp.seg_what.clear();
     bp.tables.clear();
@@ -285,7 +292,7 @@ std::string build_batch_with(BatchPlan &bp)
         // several CTAs of the one batch kernel share an SM: longer rows go multi-pass
         p.row_threads = 256;
         p.row_smem = 48 * 1024;
-        p.max_row_n = kBatchMaxRowN;
+        p.max_row_n = bp.pairs ? kPairMaxRowN : kBatchMaxRowN;
         p.max_maxe = kBatchMaxe;
         p.max_radix = bp.compact ? kCompactMaxRadix : 16;
         std::string e = build_plan_1d(p);
@@ -312,6 +319,24 @@ std::string build_batch_with(BatchPlan &bp)
             sg.dep = i == 0 ? -1 : static_cast<int>(bp.segs.size()) - 1;
             sg.ntiles = static_cast<int>(s.d.num_tiles);
             sg.fwd = s.forward ? 1 : 0;
+            if (bp.pairs) {
+                if (!s.pair) return "a segment has no pair tile";
+                PairSeg ps{};
+                ps.d = s.pd;
+                ps.in_off = sg.in_off;
+                ps.out_off = sg.out_off;
+                ps.in_buf = sg.in_buf;
+                ps.out_buf = sg.out_buf;
+                ps.dep = sg.dep;
+                bp.pair_segs.push_back(ps);
+                bp.buf_words = std::max(bp.buf_words, s.pd.buf_words);
+                const int phase = p.steps.size() == 1 ? 1 : (i == 0 ? 0 : static_cast<int>(i) + 1);
+                order.push_back({static_cast<int>(bp.segs.size()), phase, double(s.pd.n) * s.pd.P});
+                bp.segs.push_back(sg);
+                bp.segs.back().ntiles = static_cast<int>(s.pd.tiles);
+                bp.seg_what.push_back(s.what);
+                continue;
+            }
             if (s.d.tb * s.d.tpt > bp.block) return "tile shape exceeds the batch block size";
             if (s.maxe > kBatchMaxe) return "tile needs more points per thread than the batch kernel holds";
             // two buffers per CTA (the batch kernel prefetches its next item)
@@ -335,9 +360,22 @@ std::string build_batch_with(BatchPlan &bp)
     for (const Pending &pd : order)
         for (int t = 0; t < bp.segs[pd.seg].ntiles; t++) bp.items.push_back(make_int2(pd.seg, t));
     if (bp.items.size() > 0x7fffffff) return "too many tiles";
-    const int per_sm = kernel_blocks_per_sm(batch_kernel_fn(bp.forward, bp.compact), bp.block, bp.smem);
+    if (bp.pairs) {
+        bp.block = kPairThreads;
+        bp.smem = pair_smem(bp.buf_words);
+    }
+    const int per_sm = kernel_blocks_per_sm(bp.pairs ? pair_batch_fn(bp.forward) : batch_kernel_fn(bp.forward, bp.compact),
+                                            bp.block, bp.smem);
     if (per_sm <= 0) return "batch kernel does not fit on an SM";
     bp.grid = per_sm * sm_count(bp.device);
+    if (bp.pairs) {
+        const size_t pb = bp.pair_segs.size() * sizeof(PairSeg);
+        if (cudaMalloc(&bp.d_pair_segs, pb) != cudaSuccess ||
+            cudaMemcpy(bp.d_pair_segs, bp.pair_segs.data(), pb, cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaGetLastError();
+            return "twiddle table: device allocation failed";
+        }
+    }
     size_t bytes = bp.segs.size() * sizeof(BatchSeg);
     if (cudaMalloc(&bp.d_segs, bytes) != cudaSuccess ||
         cudaMemcpy(bp.d_segs, bp.segs.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -351,10 +389,20 @@ std::string build_batch_with(BatchPlan &bp)
     return std::string();
 }
 
-// The compact kernel (radices up to 10, three CTAs per SM) when every length
-// factors into them (16 and 12 split), else the kernel with every radix.
+// The pair kernel (two transforms per thread) unless a length needs a Bluestein
+// transform; then the one-transform kernels: the compact one (radices up to 10,
+// three CTAs per SM) when every length factors into them (16 and 12 split),
+// else the one with every radix.
 std::string build_batch(BatchPlan &bp)
 {
+    std::vector<int> probe;
+    bp.pairs = std::all_of(bp.sizes.begin(), bp.sizes.end(), [&](int64_t n) { return n > 1 && factor_radices(n, probe); });
+    if (bp.pairs) {
+        std::string e = build_batch_with(bp);
+        if (e != "a segment has no pair tile") return e;
+        bp.pairs = false;
+    }
+    bp.block = kBatchBlock;
     bp.compact = true;
     std::string e = build_batch_with(bp);
     if (!e.empty() && e.find("needs a radix above") != std::string::npos) {
@@ -369,6 +417,9 @@ cudaError_t enqueue(BatchPlan &bp, const void *in, void *out, void *ws, cudaStre
     cudaError_t e = cudaMemsetAsync(bp.d_counters, 0, (1 + bp.segs.size()) * sizeof(int), st);
     if (e != cudaSuccess) return e;
     BatchBufs bufs{{const_cast<void *>(in), out, ws, nullptr}};
+    if (bp.pairs)
+        return launch_pair_batch(bp.grid, bp.buf_words, bp.d_pair_segs, bp.d_items, static_cast<int>(bp.items.size()),
+                                 bp.d_counters, bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, st);
     return launch_batch(bp.grid, bp.block, bp.smem, bp.d_segs, bp.d_items, static_cast<int>(bp.items.size()),
                         bp.d_counters, bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, bp.compact,
                         st);
@@ -732,9 +783,16 @@ int64_t asdFftBatchDescribe(void *plan, char *buf, int64_t len)
     std::ostringstream o;
     o << "groups=" << bp->sizes.size() << " segments=" << bp->segs.size() << " items=" << bp->items.size()
       << " grid=" << bp->grid << " block=" << bp->block << " smem=" << bp->smem << " workspace=" << bp->ws_bytes
-      << " kernel=" << (bp->compact ? "compact radices <= 10" : "every radix") << "\n";
+      << " kernel=" << (bp->pairs ? "pairs" : (bp->compact ? "compact radices <= 10" : "every radix")) << "\n";
     for (size_t i = 0; i < bp->segs.size(); i++) {
         const auto &s = bp->segs[i];
+        if (bp->pairs) {
+            const auto &q = bp->pair_segs[i].d;
+            o << "  seg " << i << " n=" << q.n << " tiles=" << q.tiles << " pairs=" << q.P << " radices=";
+            for (int k = 0; k < q.nstages; k++) o << (k ? "x" : "") << q.st[k].R;
+            o << " dep=" << s.dep << " " << bp->seg_what[i] << "\n";
+            continue;
+        }
         o << "  seg " << i << " n=" << s.d.n << " tiles=" << s.ntiles << " tb=" << s.d.tb << " tpt=" << s.d.tpt
           << " radices=";
         for (int k = 0; k < s.d.nstages; k++) o << (k ? "x" : "") << s.d.radix[k];

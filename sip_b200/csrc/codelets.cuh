@@ -7,6 +7,13 @@
 // Constants are evaluated at compile time in double from Taylor series
 // (ccos/csin below) so no table or math-library call is needed in the
 // butterflies; every codelet is fully unrolled into FMAs on registers.
+//
+// Every codelet runs on one transform (float2) or on two at once (cpx2): the
+// kernels are bound by instruction issue, and sm_100's packed FP32 add,
+// multiply and FMA do two transforms' arithmetic in one issue slot at the
+// FP32 pipe's full rate (measured: 16 FFMA and 8 packed FMA take the same
+// pipe time in half the slots).  Both run the same operations in the same
+// order, so their results agree bit for bit.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -17,6 +24,44 @@
 
 namespace sipfft {
 
+// ---------------------------------------------------------------- packed FP32 pairs
+SIPFFT_HD float2 add2(float2 a, float2 b)
+{
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __fadd2_rn(a, b);
+#else
+    return make_float2(a.x + b.x, a.y + b.y);
+#endif
+}
+SIPFFT_HD float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+SIPFFT_HD float2 sub2(float2 a, float2 b) { return add2(a, neg2(b)); }
+SIPFFT_HD float2 mul2(float2 a, float2 b)
+{
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __fmul2_rn(a, b);
+#else
+    return make_float2(a.x * b.x, a.y * b.y);
+#endif
+}
+SIPFFT_HD float2 fma2(float2 a, float2 b, float2 c)
+{
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __ffma2_rn(a, b, c);
+#else
+    return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+#endif
+}
+SIPFFT_HD float2 both(float s) { return make_float2(s, s); }
+
+// One complex value of two transforms: re = (re 0, re 1), im = (im 0, im 1).
+struct cpx2 {
+    float2 re, im;
+};
+// interleaved complex values of the two transforms <-> cpx2
+SIPFFT_HD cpx2 pair_of(float2 a, float2 b) { return {make_float2(a.x, b.x), make_float2(a.y, b.y)}; }
+SIPFFT_HD float2 first_of(cpx2 v) { return make_float2(v.re.x, v.im.x); }
+SIPFFT_HD float2 second_of(cpx2 v) { return make_float2(v.re.y, v.im.y); }
+
 // ---------------------------------------------------------------- complex helpers
 SIPFFT_HD float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 SIPFFT_HD float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -26,18 +71,49 @@ SIPFFT_HD float2 cmul(float2 a, float2 b)
 }
 SIPFFT_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 SIPFFT_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
-// multiply by -i (FWD quarter turn) or +i
-template <bool FWD>
-SIPFFT_HD float2 mul_quarter(float2 a)
+SIPFFT_HD float2 cneg(float2 a) { return neg2(a); }
+// acc + s * a, s real
+SIPFFT_HD float2 caxpy(float s, float2 a, float2 acc) { return make_float2(fmaf(s, a.x, acc.x), fmaf(s, a.y, acc.y)); }
+// acc + i s * a, s real
+SIPFFT_HD float2 caxpy_i(float s, float2 a, float2 acc) { return make_float2(fmaf(-s, a.y, acc.x), fmaf(s, a.x, acc.y)); }
+SIPFFT_HD float2 mul_i(float2 a) { return make_float2(-a.y, a.x); }
+// a + i b, a - i b
+SIPFFT_HD float2 cadd_i(float2 a, float2 b) { return make_float2(a.x - b.y, a.y + b.x); }
+SIPFFT_HD float2 csub_i(float2 a, float2 b) { return make_float2(a.x + b.y, a.y - b.x); }
+
+SIPFFT_HD cpx2 cadd(cpx2 a, cpx2 b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
+SIPFFT_HD cpx2 csub(cpx2 a, cpx2 b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
+SIPFFT_HD cpx2 cmul(cpx2 a, cpx2 b)
 {
-    return FWD ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
+    return {fma2(a.re, b.re, neg2(mul2(a.im, b.im))), fma2(a.re, b.im, mul2(a.im, b.re))};
 }
+SIPFFT_HD cpx2 cmul(cpx2 a, float2 w) { return cmul(a, cpx2{both(w.x), both(w.y)}); }
+SIPFFT_HD cpx2 cscale(cpx2 a, float s) { return {mul2(a.re, both(s)), mul2(a.im, both(s))}; }
+SIPFFT_HD cpx2 cconj(cpx2 a) { return {a.re, neg2(a.im)}; }
+SIPFFT_HD cpx2 cneg(cpx2 a) { return {neg2(a.re), neg2(a.im)}; }
+SIPFFT_HD cpx2 caxpy(float s, cpx2 a, cpx2 acc) { return {fma2(both(s), a.re, acc.re), fma2(both(s), a.im, acc.im)}; }
+SIPFFT_HD cpx2 caxpy_i(float s, cpx2 a, cpx2 acc) { return {fma2(both(-s), a.im, acc.re), fma2(both(s), a.re, acc.im)}; }
+SIPFFT_HD cpx2 mul_i(cpx2 a) { return {neg2(a.im), a.re}; }
+SIPFFT_HD cpx2 cadd_i(cpx2 a, cpx2 b) { return {sub2(a.re, b.im), add2(a.im, b.re)}; }
+SIPFFT_HD cpx2 csub_i(cpx2 a, cpx2 b) { return {add2(a.re, b.im), sub2(a.im, b.re)}; }
+
 // exp(sign * i * theta) with the direction's sign applied to a table entry
 // that holds exp(-i * theta).
-template <bool FWD>
-SIPFFT_HD float2 dir(float2 w)
+template <bool FWD, class V>
+SIPFFT_HD V dir(V w)
 {
-    return FWD ? w : make_float2(w.x, -w.y);
+    return FWD ? w : cconj(w);
+}
+// a + w b and a - w b for a quarter turn w = -i (FWD) or +i
+template <bool FWD, class V>
+SIPFFT_HD V add_quarter(V a, V b)
+{
+    return FWD ? csub_i(a, b) : cadd_i(a, b);
+}
+template <bool FWD, class V>
+SIPFFT_HD V sub_quarter(V a, V b)
+{
+    return FWD ? cadd_i(a, b) : csub_i(a, b);
 }
 
 // ---------------------------------------------------------------- compile-time trig
@@ -77,23 +153,42 @@ struct Root {
     static constexpr float s = static_cast<float>(csin(2.0 * kPi * (J % R) / R));
 };
 
+// e + w a and e - w a, w = exp(-+ 2*pi*i*J/R) = c + i s, in six FMAs: with |c| >= |s|
+// as e +- c u, u = a + i (s/c) a, else as e +- s u, u = (c/s) a + i a (two
+// roundings a component instead of the three of product, sum and butterfly).
+template <int R, int J, bool FWD, class V>
+SIPFFT_HD void rot_butterfly(V e, V a, V &plus, V &minus)
+{
+    constexpr double t = 2.0 * kPi * (J % R) / R;
+    constexpr double c = ccos(t), s = FWD ? -csin(t) : csin(t);
+    constexpr bool wide = (c < 0 ? -c : c) >= (s < 0 ? -s : s);
+    V u;
+    if constexpr (wide)
+        u = caxpy_i(static_cast<float>(s / c), a, a);
+    else
+        u = caxpy(static_cast<float>(c / s), a, mul_i(a));
+    constexpr float m = static_cast<float>(wide ? c : s);
+    plus = caxpy(m, u, e);
+    minus = caxpy(-m, u, e);
+}
+
 // multiply a by exp(-+ 2*pi*i*J/R) with the trivial angles special-cased
-template <int R, int J, bool FWD>
-SIPFFT_HD float2 rot(float2 a)
+template <int R, int J, bool FWD, class V>
+SIPFFT_HD V rot(V a)
 {
     constexpr int j = ((J % R) + R) % R;
     if constexpr (j == 0) {
         return a;
     } else if constexpr (4 * j == R) {
-        return mul_quarter<FWD>(a);
+        return FWD ? cneg(mul_i(a)) : mul_i(a);
     } else if constexpr (2 * j == R) {
-        return make_float2(-a.x, -a.y);
+        return cneg(a);
     } else if constexpr (4 * j == 3 * R) {
-        return mul_quarter<!FWD>(a);
+        return FWD ? mul_i(a) : cneg(mul_i(a));
     } else {
         constexpr float c = Root<R, j>::c;
         constexpr float s = FWD ? -Root<R, j>::s : Root<R, j>::s;  // exp(+-i theta) = c + i*s
-        return make_float2(fmaf(a.x, c, -a.y * s), fmaf(a.x, s, a.y * c));
+        return cmul(a, make_float2(c, s));
     }
 }
 
@@ -101,9 +196,10 @@ SIPFFT_HD float2 rot(float2 a)
 // Recursive radix-2 decimation in time on an array held in registers.
 template <int R, bool FWD>
 struct Pow2 {
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
-        float2 e[R / 2], o[R / 2];
+        V e[R / 2], o[R / 2];
 #pragma unroll
         for (int i = 0; i < R / 2; i++) {
             e[i] = a[2 * i];
@@ -113,40 +209,51 @@ struct Pow2 {
         Pow2<R / 2, FWD>::run(o);
         combine<0>(a, e, o);
     }
-    template <int K>
-    SIPFFT_HD static void combine(float2 *a, const float2 *e, const float2 *o)
+    template <int K, class V>
+    SIPFFT_HD static void combine(V *a, const V *e, const V *o)
     {
         if constexpr (K < R / 2) {
-            float2 t = rot<R, K, FWD>(o[K]);
-            a[K] = cadd(e[K], t);
-            a[K + R / 2] = csub(e[K], t);
+            if constexpr (4 * K == R) {
+                a[K] = add_quarter<FWD>(e[K], o[K]);
+                a[K + R / 2] = sub_quarter<FWD>(e[K], o[K]);
+            } else if constexpr (K == 0) {
+                a[0] = cadd(e[0], o[0]);
+                a[R / 2] = csub(e[0], o[0]);
+            } else {
+                rot_butterfly<R, K, FWD>(e[K], o[K], a[K], a[K + R / 2]);
+            }
             combine<K + 1>(a, e, o);
         }
     }
 };
 template <bool FWD>
 struct Pow2<1, FWD> {
-    SIPFFT_HD static void run(float2 *) {}
+    template <class V>
+    SIPFFT_HD static void run(V *)
+    {
+    }
 };
 template <bool FWD>
 struct Pow2<2, FWD> {
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
-        float2 t = a[1];
+        const V t = a[1];
         a[1] = csub(a[0], t);
         a[0] = cadd(a[0], t);
     }
 };
 template <bool FWD>
 struct Pow2<4, FWD> {
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
-        float2 t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
-        float2 t2 = cadd(a[1], a[3]), t3 = mul_quarter<FWD>(csub(a[1], a[3]));
+        const V t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
+        const V t2 = cadd(a[1], a[3]), t3 = csub(a[1], a[3]);
         a[0] = cadd(t0, t2);
         a[2] = csub(t0, t2);
-        a[1] = cadd(t1, t3);
-        a[3] = csub(t1, t3);
+        a[1] = add_quarter<FWD>(t1, t3);
+        a[3] = sub_quarter<FWD>(t1, t3);
     }
 };
 
@@ -158,51 +265,42 @@ struct Pow2<4, FWD> {
 template <int R, bool FWD>
 struct Odd {
     static constexpr int H = (R - 1) / 2;
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
-        float2 tp[H], tm[H];
+        V tp[H], tm[H];
 #pragma unroll
         for (int k = 1; k <= H; k++) {
             tp[k - 1] = cadd(a[k], a[R - k]);
             tm[k - 1] = csub(a[k], a[R - k]);
         }
-        float2 y0 = a[0];
+        V y0 = a[0];
 #pragma unroll
         for (int k = 0; k < H; k++) y0 = cadd(y0, tp[k]);
-        float2 out[R];
+        V out[R];
         out[0] = y0;
         terms<1>(a[0], tp, tm, out);
 #pragma unroll
         for (int i = 0; i < R; i++) a[i] = out[i];
     }
-    template <int M>
-    SIPFFT_HD static void terms(float2 a0, const float2 *tp, const float2 *tm, float2 *out)
+    template <int M, class V>
+    SIPFFT_HD static void terms(V a0, const V *tp, const V *tm, V *out)
     {
         if constexpr (M <= H) {
-            float2 b = a0, d = make_float2(0.f, 0.f);
+            V b = a0, d = cscale(tm[0], Root<R, M % R>::s);
             accum<M, 1>(b, d, tp, tm);
             // forward: y_M = b - i d ; y_{R-M} = b + i d
-            float2 id = make_float2(-d.y, d.x);  // i*d
-            if constexpr (FWD) {
-                out[M] = csub(b, id);
-                out[R - M] = cadd(b, id);
-            } else {
-                out[M] = cadd(b, id);
-                out[R - M] = csub(b, id);
-            }
+            out[M] = add_quarter<FWD>(b, d);
+            out[R - M] = sub_quarter<FWD>(b, d);
             terms<M + 1>(a0, tp, tm, out);
         }
     }
-    template <int M, int K>
-    SIPFFT_HD static void accum(float2 &b, float2 &d, const float2 *tp, const float2 *tm)
+    template <int M, int K, class V>
+    SIPFFT_HD static void accum(V &b, V &d, const V *tp, const V *tm)
     {
         if constexpr (K <= H) {
-            constexpr float c = Root<R, (K * M) % R>::c;
-            constexpr float s = Root<R, (K * M) % R>::s;
-            b.x = fmaf(c, tp[K - 1].x, b.x);
-            b.y = fmaf(c, tp[K - 1].y, b.y);
-            d.x = fmaf(s, tm[K - 1].x, d.x);
-            d.y = fmaf(s, tm[K - 1].y, d.y);
+            b = caxpy(Root<R, (K * M) % R>::c, tp[K - 1], b);
+            if constexpr (K > 1) d = caxpy(Root<R, (K * M) % R>::s, tm[K - 1], d);
             accum<M, K + 1>(b, d, tp, tm);
         }
     }
@@ -210,23 +308,17 @@ struct Odd {
 
 template <bool FWD>
 struct Odd<3, FWD> {
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
         constexpr float h = 0.86602540378443864676f;  // sqrt(3)/2
-        float2 s = cadd(a[1], a[2]);
-        float2 d = csub(a[1], a[2]);
-        float2 y0 = cadd(a[0], s);
-        float2 m = make_float2(fmaf(-0.5f, s.x, a[0].x), fmaf(-0.5f, s.y, a[0].y));
+        const V s = cadd(a[1], a[2]);
+        const V d = csub(a[1], a[2]);
+        const V m = caxpy(-0.5f, s, a[0]);
+        a[0] = cadd(a[0], s);
         // forward: y1 = m - i h d, y2 = m + i h d
-        float2 ihd = make_float2(-h * d.y, h * d.x);
-        a[0] = y0;
-        if (FWD) {
-            a[1] = csub(m, ihd);
-            a[2] = cadd(m, ihd);
-        } else {
-            a[1] = cadd(m, ihd);
-            a[2] = csub(m, ihd);
-        }
+        a[1] = caxpy_i(FWD ? -h : h, d, m);
+        a[2] = caxpy_i(FWD ? h : -h, d, m);
     }
 };
 
@@ -252,8 +344,8 @@ constexpr int comp_first(int r)
     return smallest_prime_factor(r);
 }
 
-template <int R, bool FWD>
-SIPFFT_HD void dft(float2 *a);
+template <int R, bool FWD, class V>
+SIPFFT_HD void dft(V *a);
 
 // Composite radix R = A*B in registers (Cooley-Tukey, decimation in time):
 // B-point DFTs over the A interleaved sub-sequences, twiddles W_R^(n1*k2),
@@ -261,9 +353,10 @@ SIPFFT_HD void dft(float2 *a);
 template <int A, int B, bool FWD>
 struct Comp {
     static constexpr int R = A * B;
-    SIPFFT_HD static void run(float2 *a)
+    template <class V>
+    SIPFFT_HD static void run(V *a)
     {
-        float2 y[A][B];
+        V y[A][B];
 #pragma unroll
         for (int n1 = 0; n1 < A; n1++) {
 #pragma unroll
@@ -273,7 +366,7 @@ struct Comp {
         twiddle<1, 1>(y);
 #pragma unroll
         for (int k2 = 0; k2 < B; k2++) {
-            float2 z[A];
+            V z[A];
 #pragma unroll
             for (int n1 = 0; n1 < A; n1++) z[n1] = y[n1][k2];
             dft<A, FWD>(z);
@@ -281,8 +374,8 @@ struct Comp {
             for (int k1 = 0; k1 < A; k1++) a[k2 + B * k1] = z[k1];
         }
     }
-    template <int N1, int K2>
-    SIPFFT_HD static void twiddle(float2 (&y)[A][B])
+    template <int N1, int K2, class V>
+    SIPFFT_HD static void twiddle(V (&y)[A][B])
     {
         if constexpr (N1 < A) {
             if constexpr (K2 < B) {
@@ -295,8 +388,8 @@ struct Comp {
     }
 };
 
-template <int R, bool FWD>
-SIPFFT_HD void dft(float2 *a)
+template <int R, bool FWD, class V>
+SIPFFT_HD void dft(V *a)
 {
     if constexpr (is_pow2<R>()) {
         Pow2<R, FWD>::run(a);

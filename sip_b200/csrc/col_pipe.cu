@@ -5,23 +5,24 @@
 // columns of an [outer][n][cols] array.  The tensor-memory-access engine
 // copies it into shared memory as 3D boxes of TB columns x up to 256 rows
 // (one rectangular copy per 256 rows, issued by one thread and completed on
-// an mbarrier), double-buffered so that the next tile streams in while the
-// current one is transformed.  The first Stockham stage reads the staged rows
-// column by column (applying a multi-pass step's inter-pass twiddles), the
-// stages run in the padded work rows that overwrite the staging buffer, and
-// the last stage stores straight from registers to HBM (TB consecutive threads
-// write TB consecutive columns of one row).  The reference runs this axis as
+// an mbarrier).  A thread transforms two adjacent columns at once (cpx2: a
+// 16-byte word of the staged tile holds both), so that index arithmetic,
+// shared-memory accesses and twiddle loads are paid once for two columns and
+// the butterflies run as packed FP32 instructions; the last stage stores
+// straight from registers to HBM, 16 bytes a thread where the columns are
+// adjacent there as well.  The reference runs this axis as
 // a transpose plus a DFT-matrix GEMM (core/fft/fftcore/fft_core_stride.cpp:36-188,
 // ops/fft/c2c/fft_stride/fft_stride/kernel/fft_stride.cce) or as explicit
 // Transpose steps around the row cores (core/fft/fft_api.cpp:527-697).
 //
 // Launch preconditions (the planner checks them, the exec path re-checks the
 // pointer): source 16-byte aligned, column stride 1, element and outer
-// strides multiples of 2 complex values (16 bytes), TB even.
+// strides multiples of 2 complex values (16 bytes), column and tile counts
+// below 2^31.
 #include <cuda.h>
 
 #include "sipfft_internal.h"
-#include "static_engine.cuh"
+#include "pair_engine.cuh"
 
 namespace sipfft {
 
@@ -37,54 +38,44 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// element e of column l of the staged tile ([row][TB] dense), with the
-// inter-pass twiddle of a multi-pass step applied on read
-template <int TB, bool FWD>
-struct ColStage {
-    const float2 *tile;
-    int l;
-    const TileDesc *d;
-    int64_t kc;  // Stockham column of the pass twiddle, < 0 for none
-    __device__ __forceinline__ float2 operator()(int e) const
-    {
-        const float2 v = tile[e * TB + l];
-        return kc >= 0 ? cmul(v, pass_twiddle<FWD>(*d, e, kc)) : v;
-    }
-};
-
-struct ColOut {
-    float2 *col;
-    int64_t es;
-    __device__ __forceinline__ void operator()(int e, float2 v) const { st_stream(col + e * es, v); }
-};
-
 }  // namespace
 
-// PP: a third shared-memory buffer holds the even stage boundaries (ping-pong
-// work rows), so stage 0 scatters outside the staged tile and no stage needs a
-// barrier between its gather and its scatter.
-// COUT: each column's N outputs are contiguous (output element stride 1, the
-// first pass of a multi-pass transform): the last stage writes the work rows and
-// the CTA then stores whole column runs, a warp 32 consecutive elements instead
-// of 16 columns x 2.
-template <class Q, int T, int TB, bool PP, bool COUT, bool FWD>
-__global__ void __launch_bounds__(TB *T, (TB * T <= 256) ? 3 : 1)
+// Shared memory of one CTA: barriers, two tile buffers, and with PP a work tile.
+// COUT: contiguous column outputs (pair_last_runs).
+template <class Q, int T, int P, bool PP, bool COUT>
+struct ColShape {
+    using Tile = PairTile<Q, P, COUT ? P + 1 : P>;
+    static constexpr int kThreads = P * T;
+    static constexpr int kTileWords = P * Q::N;  // 16-byte words
+    static constexpr int kBufWords = PP || Tile::kWords < kTileWords ? kTileWords : Tile::kWords;
+    static constexpr size_t kSmem = 128 + (size_t(2) * kBufWords + (PP ? Tile::kWords : 0)) * sizeof(float4);
+    static constexpr int kPerSm = static_cast<int>(size_t(228 * 1024) / (kSmem + 1024));
+    static_assert(kPerSm >= 1 && Q::N / T == 16 && kBufWords % 8 == 0, "tile shape");
+};
+
+// Two tile buffers: the next tile streams into one while the other is
+// transformed.  The work tile takes the staged tile's place once stage 0 has
+// read it; with PP (2048 points, one CTA per SM) it has memory of its own, which
+// saves the barrier in between.  Measured on 65536 x 256: a staging tile of its
+// own, refilled after stage 0, left too few bytes in flight.
+template <class Q, int T, int P, bool PP, bool COUT, bool FWD>
+__global__ void __launch_bounds__(ColShape<Q, T, P, PP, COUT>::kThreads, ColShape<Q, T, P, PP, COUT>::kPerSm)
     col_pipe_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ TileDesc d, int *err)
 {
     pdl_enter();
-    using E = StaticEngine<Q, T, Pads<>, PP>;
-    constexpr int N = Q::N;
+    using Shape = ColShape<Q, T, P, PP, COUT>;
+    using Tile = typename Shape::Tile;
+    constexpr int N = Q::N, TB = 2 * P;
     constexpr int BOX = N < 256 ? N : 256;
     constexpr int NBOX = N / BOX;
-    constexpr uint32_t kTileBytes = uint32_t(TB) * N * sizeof(float2);
     extern __shared__ __align__(128) unsigned char smraw[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smraw);
-    float2 *bufs = reinterpret_cast<float2 *>(smraw + 128);
-    const int64_t buf_f2 = d.col_buf;  // per-buffer float2 count (planner-computed)
+    float4 *bufs = reinterpret_cast<float4 *>(smraw + 128);
     const int tid = threadIdx.x;
-    const int l = tid % TB, lane = tid / TB;
+    const int p = tid % P, lane = tid / P;
     float2 *out = static_cast<float2 *>(d.out);
-    __shared__ int64_t s_base[COUT ? TB : 1];  // output offsets of the tile's columns (COUT)
+    const uint32_t tiles = static_cast<uint32_t>(d.num_tiles);
+    const uint32_t cols = static_cast<uint32_t>(d.n_cols);
 
     if (tid == 0) {
         mbar_init(&bars[0], 1);
@@ -93,52 +84,58 @@ __global__ void __launch_bounds__(TB *T, (TB * T <= 256) ? 3 : 1)
     }
     __syncthreads();
 
-    auto issue = [&](int64_t t, int b) {
+    auto issue = [&](uint32_t t, int b) {
         if (tid == 0) {
-            const int o = static_cast<int>(t / d.tiles_per_outer);
-            const int c0 = static_cast<int>((t % d.tiles_per_outer) * TB);
-            float2 *dst = bufs + b * buf_f2;
+            const uint32_t o = d.dv_tiles.div(t), c0 = (t - o * d.dv_tiles.d) * TB;
+            float4 *dst = bufs + b * Shape::kBufWords;
             fence_proxy_async_smem();
-            mbar_arrive_expect_tx(&bars[b], kTileBytes);
+            mbar_arrive_expect_tx(&bars[b], static_cast<uint32_t>(Shape::kTileWords * sizeof(float4)));
 #pragma unroll
-            for (int k = 0; k < NBOX; k++) tma_load_3d(dst + k * BOX * TB, &tmap, c0, k * BOX, o, &bars[b]);
+            for (int k = 0; k < NBOX; k++)
+                tma_load_3d(dst + k * BOX * P, &tmap, static_cast<int>(c0), k * BOX, static_cast<int>(o), &bars[b]);
         }
     };
 
-    int64_t t = blockIdx.x;
-    if (t < d.num_tiles) issue(t, 0);
-    for (int i = 0; t < d.num_tiles; t += gridDim.x, i++) {
+    uint32_t t = blockIdx.x;
+    if (t < tiles) issue(t, 0);
+    for (int i = 0; t < tiles; t += gridDim.x, i++) {
         const int b = i & 1;
-        const int64_t tn = t + gridDim.x;
-        if (tn < d.num_tiles) issue(tn, b ^ 1);
+        const uint32_t tn = t + gridDim.x;
+        if (tn < tiles) issue(tn, b ^ 1);
         // a thread whose bounded wait gave up still runs the tile (every access
         // stays in bounds) and the CTA leaves together at the end of the iteration
         const bool timed_out = !mbar_wait_bounded(&bars[b], (i >> 1) & 1);
         if (timed_out) atomicExch(err, 1);
-        const int64_t o = t / d.tiles_per_outer;
-        const int64_t c0 = (t % d.tiles_per_outer) * TB;
-        const int64_t left = d.n_cols - c0;
-        const bool active = l < left;
-        float2 *buf = bufs + b * buf_f2;
-        float2 *work2 = PP ? bufs + 2 * buf_f2 + l * d.pitch : nullptr;
-        const int64_t kc = d.g_twiddle ? pass_column(d, c0 + l) : -1;
-        if constexpr (COUT) {
-            if (tid < TB) s_base[tid] = col_base(d.out_a, o, c0 + tid);
-            E::template run<FWD>(d, buf + l * d.pitch, ColStage<TB, FWD>{buf, l, &d, kc}, SmemRow{buf + l * d.pitch},
-                                 true, lane, active, work2);
-            __syncthreads();
-            const int cols = left < TB ? static_cast<int>(left) : TB;
-            for (int c = 0; c < cols; c++) {
-                float2 *dst = out + s_base[c];
-                const float2 *src = buf + c * d.pitch;
-                for (int e = tid; e < N; e += TB * T) st_stream(dst + e, src[pad(e)]);
-            }
-        } else {
-            E::template run<FWD>(d, buf + l * d.pitch, ColStage<TB, FWD>{buf, l, &d, kc},
-                                 ColOut{out + col_base(d.out_a, o, c0 + l), d.out_a.estride}, false, lane, active,
-                                 work2);
+        const uint32_t o = d.dv_tiles.div(t), ct = (t - o * d.dv_tiles.d) * TB, c0 = ct + 2 * p;
+        PassTwiddle tw{nullptr, nullptr, 0, 0, 0};
+        if (d.g_twiddle) {
+            tw.t1 = d.g_t1;
+            tw.t2 = d.g_t2;
+            tw.ns = d.dv_gns.d;
+            tw.k0 = d.dv_gns.mod(d.dv_gdiv.div(c0));
+            tw.k1 = d.dv_gns.mod(d.dv_gdiv.div(c0 + 1));
         }
-        // buffer b is free for the copy issued in iteration i+1; a CTA-uniform exit after a timeout
+        float4 *buf = bufs + b * Shape::kBufWords;
+        float4 *work = PP ? bufs + 2 * Shape::kBufWords : buf;
+        cpx2 v[static_maxv<Q, T>()];
+        pair_stage0<Q, T, P, FWD>(v, buf + p, lane, tw,
+                                  PassTable2{d.g_lo, d.g_hi, d.g_log2l, static_cast<uint32_t>(d.g_step)});
+        if constexpr (!PP) __syncthreads();
+        sscatter<Q, 0, T>(v, typename Tile::template Row<0>{work + p}, lane, true);
+        __syncthreads();
+        if constexpr (COUT) {
+            pair_last_runs<Q, T, P, P + 1, FWD>(
+                v, work, tid, cols - ct,
+                [&](int c) { return out + col_base32(d.out_a, d.dv_block, o, ct + c); }, d.stw);
+        } else {
+            const int64_t b0 = col_base32(d.out_a, d.dv_block, o, c0), b1 = col_base32(d.out_a, d.dv_block, o, c0 + 1);
+            const bool wide = b1 == b0 + 1 && ((reinterpret_cast<uintptr_t>(out + b0) & 15) == 0) &&
+                              d.out_a.estride % 2 == 0 && c0 + 1 < cols;
+            pair_stages<Q, T, P, FWD, 1>(v, work + p,
+                                         PairColumns{out + b0, out + b1, d.out_a.estride, c0 + 1 < cols, wide}, lane,
+                                         c0 < cols, d.stw);
+        }
+        // the buffers are free for the copy issued in iteration i+1; a CTA-uniform exit after a timeout
         if (__syncthreads_or(timed_out)) return;
     }
 }
@@ -147,37 +144,37 @@ __global__ void __launch_bounds__(TB *T, (TB * T <= 256) ? 3 : 1)
 namespace {
 
 struct ColPipeEntry {
-    int n, tpt, tb, bufs;  // bufs: shared-memory buffers of col_buf float2 each (3: ping-pong work rows)
+    int n, tpt, tb;
+    size_t smem[2];
+    int nstages, radix[4];
     const void *fn[2][2];  // [contiguous column outputs][forward]
 };
 
-template <class Q, int T, int TB, bool PP = false>
+template <class Q, int T, int P, bool PP = false>
 ColPipeEntry col_entry()
 {
-    static_assert(TB % 2 == 0 && TB * T <= 512, "column tile shape");
-    ColPipeEntry e{Q::N, T, TB, PP ? 3 : 2,
-                   {{reinterpret_cast<const void *>(col_pipe_kernel<Q, T, TB, PP, false, false>),
-                     reinterpret_cast<const void *>(col_pipe_kernel<Q, T, TB, PP, false, true>)},
+    ColPipeEntry e{Q::N, T, 2 * P, {ColShape<Q, T, P, PP, false>::kSmem, 0}, Q::S, {},
+                   {{reinterpret_cast<const void *>(col_pipe_kernel<Q, T, P, PP, false, false>),
+                     reinterpret_cast<const void *>(col_pipe_kernel<Q, T, P, PP, false, true>)},
                     {nullptr, nullptr}}};
-    // staged contiguous-column stores pay off where a warp's direct stores would
-    // cover less than a 32-byte sector of each column (TB >= 16: two lanes, 16 bytes)
-    if constexpr (TB >= 16) {
-        e.fn[1][0] = reinterpret_cast<const void *>(col_pipe_kernel<Q, T, TB, PP, true, false>);
-        e.fn[1][1] = reinterpret_cast<const void *>(col_pipe_kernel<Q, T, TB, PP, true, true>);
+    for (int s = 0; s < Q::S; s++) e.radix[s] = Q::r[s];
+    if constexpr (P >= 8 && Q::S == 2) {
+        e.smem[1] = ColShape<Q, T, P, PP, true>::kSmem;
+        e.fn[1][0] = reinterpret_cast<const void *>(col_pipe_kernel<Q, T, P, PP, true, false>);
+        e.fn[1][1] = reinterpret_cast<const void *>(col_pipe_kernel<Q, T, P, PP, true, true>);
     }
     return e;
 }
 
-// Engines with 16 points per thread (the same radix sequences as the
-// power-of-two row engines); TB columns per tile as the planner chooses them
-// (CTAs of at most 256 threads, three per SM, while TB stays >= 4, i.e. rows
-// of at least one 32-byte sector; 512 threads for 2048 points, one CTA per SM,
-// whose shared memory also holds the ping-pong work rows).
+// Engines with 16 points of two columns per thread.  Tiles of 32 KB (16 KB for
+// 64 points), 64 and 128 threads: three to six CTAs per SM and up to 168
+// registers a thread; 128-byte row runs up to 256 points, 64 and 32 bytes for
+// 512 and 1024 points.  2048 points: 64 KB tiles, one CTA of 256 threads.
 const std::vector<ColPipeEntry> &col_registry()
 {
     static const std::vector<ColPipeEntry> r = {
-        col_entry<Seq<16, 4>, 4, 16>(),     col_entry<Seq<16, 8>, 8, 16>(),   col_entry<Seq<16, 16>, 16, 16>(),
-        col_entry<Seq<16, 16, 2>, 32, 8>(), col_entry<Seq<16, 16, 4>, 64, 4>(), col_entry<Seq<16, 16, 8>, 128, 4, true>(),
+        col_entry<Seq<16, 4>, 4, 16>(),     col_entry<Seq<16, 8>, 8, 16>(),    col_entry<Seq<16, 16>, 16, 8>(),
+        col_entry<Seq<16, 16, 2>, 32, 4>(), col_entry<Seq<16, 16, 4>, 64, 2>(), col_entry<Seq<16, 16, 8>, 128, 2, true>(),
     };
     return r;
 }
@@ -203,52 +200,43 @@ EncodeTiledFn encode_fn()
 
 }  // namespace
 
-const void *col_pipe_kernel_fn(int n, int tpt, int tb, bool forward, bool contiguous_out)
+bool col_pipe_kernel(int n, bool forward, bool contiguous_out, ColPipe &c)
 {
     for (const ColPipeEntry &e : col_registry())
-        if (e.n == n && e.tpt == tpt && e.tb == tb) {
-            const int f = forward ? 1 : 0;
-            return contiguous_out && e.fn[1][f] ? e.fn[1][f] : e.fn[0][f];
+        if (e.n == n) {
+            const int k = contiguous_out && e.fn[1][0] ? 1 : 0;
+            c = ColPipe{e.fn[k][forward ? 1 : 0], e.tpt, e.tb, e.smem[k], e.nstages,
+                        {e.radix[0], e.radix[1], e.radix[2], e.radix[3]}};
+            return true;
         }
-    return nullptr;
-}
-
-int col_pipe_bufs(int n, int tpt, int tb)
-{
-    for (const ColPipeEntry &e : col_registry())
-        if (e.n == n && e.tpt == tpt && e.tb == tb) return e.bufs;
-    return 2;
+    return false;
 }
 
 bool col_pipe_has_engine(int n)
 {
-    for (const ColPipeEntry &e : col_registry())
-        if (e.n == n) return true;
-    return false;
+    ColPipe c;
+    return col_pipe_kernel(n, true, false, c);
 }
 
 void col_pipe_kernel_fns(std::vector<const void *> &out)
 {
     for (const ColPipeEntry &e : col_registry())
-        for (int c = 0; c < 2; c++)
+        for (int k = 0; k < 2; k++)
             for (int f = 0; f < 2; f++)
-                if (e.fn[c][f]) out.push_back(e.fn[c][f]);
+                if (e.fn[k][f]) out.push_back(e.fn[k][f]);
 }
 
-size_t col_pipe_smem(const TileDesc &d)
-{
-    return 128 + (d.row_bufs == 3 ? 3 : 2) * static_cast<size_t>(d.col_buf) * sizeof(float2);
-}
-
+// At least half a tile of columns: below that the element-copy tiles waste less.
 bool col_pipe_layout_ok(const TileDesc &d)
 {
     const Addr &a = d.in_a;
-    return d.tb % 2 == 0 && d.n_cols >= d.tb && a.cstride == 1 && a.cblock == 0 && a.estride % 2 == 0 && a.estride > 0 &&
-           (d.n_outer == 1 || a.dist % 2 == 0) && d.n_outer < (int64_t(1) << 31) &&
-           d.tiles_per_outer * d.tb < (int64_t(1) << 31) && encode_fn() != nullptr;
+    const int64_t most = int64_t(1) << 31;
+    return 2 * d.n_cols >= d.tb && a.cstride == 1 && a.cblock == 0 && a.estride % 2 == 0 && a.estride > 0 &&
+           (d.n_outer == 1 || a.dist % 2 == 0) && d.n_outer < most && d.tiles_per_outer * d.tb < most &&
+           d.num_tiles < most && d.out_a.cblock < most && d.g_div < most && d.g_ns < most && encode_fn() != nullptr;
 }
 
-cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, int grid, int *err, cudaStream_t st)
+cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, size_t smem, int grid, int *err, cudaStream_t st)
 {
     if (!fn || grid <= 0 || (reinterpret_cast<uintptr_t>(d.in) & 15)) return cudaErrorInvalidConfiguration;
     EncodeTiledFn enc = encode_fn();
@@ -270,7 +258,7 @@ cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, int grid, int *er
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     TileDesc dd = d;
     void *args[] = {&map, &dd, &err};
-    return launch_pdl(fn, dim3(grid), dim3(d.tb * d.tpt), col_pipe_smem(d), st, args);
+    return launch_pdl(fn, dim3(grid), dim3(d.tb / 2 * d.tpt), smem, st, args);
 }
 
 }  // namespace sipfft

@@ -392,6 +392,26 @@ __global__ void twiddle_kernel(float2 *t, int64_t count, int64_t denom, int64_t 
     }
 }
 
+// t[j * ns + k] = exp(-2 pi i j k / denom), the same way
+__global__ void outer_twiddle_kernel(float2 *t, int64_t count, int64_t ns, int64_t denom)
+{
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count;
+         i += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t idx = (i / ns) * (i % ns) % denom;
+        double s, c;
+        sincospi(2.0 * static_cast<double>(idx) / static_cast<double>(denom), &s, &c);
+        t[i] = make_float2(static_cast<float>(c), static_cast<float>(-s));
+    }
+}
+
+cudaError_t fill_outer_twiddles(float2 *t, int64_t rows, int64_t ns, int64_t denom, cudaStream_t st)
+{
+    const int64_t count = rows * ns;
+    const int grid = static_cast<int>(std::min<int64_t>((count + 255) / 256, 4096));
+    outer_twiddle_kernel<<<grid, 256, 0, st>>>(t, count, ns, denom);
+    return cudaGetLastError();
+}
+
 // Bluestein tables.  chirp[n] = exp(s*pi*i*(n^2 mod 2N)/N) (s = -1 forward),
 // with n^2 reduced exactly in 64-bit integers before the FP64 evaluation.
 __global__ void chirp_kernel(float2 *t, int64_t n_len, int sign)

@@ -61,6 +61,30 @@ __host__ __device__ constexpr uint32_t ns_reciprocal(int ns)
     return ns <= 1 ? 0u : static_cast<uint32_t>(((uint64_t(1) << 32) + uint64_t(ns) - 1) / uint64_t(ns));
 }
 
+// Division of n < 2^31 by a fixed divisor 1 <= d < 2^31 as a multiply and a
+// shift: mul = floor(2^(31+l) / d) + 1 with l = ceil(log2 d), q = hi32(n mul) >> (l-1).
+struct FastDiv {
+    uint32_t d, mul, shift;  // d = 1: mul = 0
+    __host__ __device__ __forceinline__ uint32_t div(uint32_t n) const
+    {
+        if (mul == 0) return n;
+#ifdef __CUDA_ARCH__
+        return __umulhi(n, mul) >> shift;
+#else
+        return static_cast<uint32_t>((uint64_t(n) * mul) >> 32) >> shift;
+#endif
+    }
+    __host__ __device__ __forceinline__ uint32_t mod(uint32_t n) const { return n - div(n) * d; }
+};
+inline FastDiv fast_div(int64_t d)
+{
+    if (d <= 1) return FastDiv{1, 0, 0};
+    int l = 0;
+    while ((int64_t(1) << l) < d) l++;
+    return FastDiv{static_cast<uint32_t>(d), static_cast<uint32_t>((uint64_t(1) << (31 + l)) / static_cast<uint64_t>(d) + 1),
+                   static_cast<uint32_t>(l - 1)};
+}
+
 struct TileDesc {
     const void *in;
     void *out;
@@ -114,18 +138,21 @@ struct TileDesc {
     int planar;
     const float *in_im;
     float *out_im;
-    // Shared-memory buffers of a row kernel, each g_ns float2 (of a TMA column
-    // kernel: each col_buf float2): 2 (double-buffered tiles; 0 reads as 2) or
-    // 3 (plus a ping-pong work area).
+    // Shared-memory buffers of a row kernel, each g_ns float2: 2 (double-buffered
+    // tiles; 0 reads as 2) or 3 (plus a ping-pong work area).
     int row_bufs;
     // complex32 (FP16 real / imaginary pairs) user data of a C2C step: bit 0 =
     // the input, bit 1 = the output.  Loads widen to FP32, the stages run in
     // FP32, stores round to FP16 (round to nearest even).
     int half_io;
-    // Shared-memory float2 count of one tile buffer of the TMA column kernel
-    // (col_pipe.cu): >= tb * max(n, pitch), a multiple of 16 (128-byte aligned
-    // buffers).
-    int64_t col_buf;
+    // The same input twiddle for the column kernels, as t1[j][k] t2[r][k] of
+    // element j + r n/radix[0] and Stockham column k (rows of g_ns entries);
+    // t1 null: from the two-level table.
+    const float2 *g_t1;
+    const float2 *g_t2;
+    // Divisors of the column kernels' 32-bit index arithmetic: tiles_per_outer,
+    // out_a.cblock, g_div, g_ns (each 1 where unused).
+    FastDiv dv_tiles, dv_block, dv_gdiv, dv_gns;
 };
 
 // Stockham column of tile column c for the pass twiddle: (c / g_div) mod g_ns.

@@ -13,7 +13,9 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <mutex>
 #include <sstream>
+#include <tuple>
 
 #include "sipfft_internal.h"
 
@@ -171,6 +173,82 @@ bool split_passes(int64_t n, int parts, std::vector<int> &out)
     return true;
 }
 
+// Radices (2..16, the largest first: longer contiguous runs in the last stage,
+// shorter pass tables) and pairs of the cheapest pair tile of length n
+// (pair_tile_cost), at most max_pairs pairs; cost 1e30 when none fits.
+struct PairChoice {
+    double cost = 1e30;
+    std::vector<int> radices;
+    int P = 0;
+};
+struct PairSearch {
+    int n;
+    bool rows, runs;
+    int64_t raw_dist;
+    int max_pairs;
+    PairChoice best;
+    std::vector<int> cur;
+    void leaf()
+    {
+        PairDesc q{};
+        const int S = static_cast<int>(cur.size());
+        for (int P = max_pairs; P >= 1; P = rows ? P - 1 : P / 2) {
+            if (!pair_shape(q, n, cur.data(), S, rows, runs, raw_dist, P)) continue;
+            const double c = pair_tile_cost(n, cur.data(), S, rows, P, q.buf_words);
+            if (c < best.cost) {
+                best.cost = c;
+                best.radices = cur;
+                best.P = P;
+            }
+            if (!rows) break;  // fewer columns never pay
+        }
+    }
+    void walk(int m, int most, int stages_left)
+    {
+        if (m == 1) return leaf();
+        if (stages_left == 0) return;
+        for (int R = std::min(most, m); R >= 2; R--) {
+            if (m % R) continue;
+            cur.push_back(R);
+            walk(m / R, R, stages_left - 1);
+            cur.pop_back();
+        }
+    }
+};
+PairChoice pair_choice(int n, bool rows, bool runs, int64_t raw_dist, int max_pairs)
+{
+    static std::mutex mu;
+    static std::map<std::tuple<int, bool, bool, int64_t, int>, PairChoice> memo;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(n, rows, runs, raw_dist, max_pairs);
+    auto it = memo.find(key);
+    if (it != memo.end()) return it->second;
+    PairSearch s{n, rows, runs, raw_dist, max_pairs, {}, {}};
+    // the fewest stages that reach n, and one more
+    int fewest = 1;
+    for (int64_t m = 16; m < n; m *= 16) fewest++;
+    for (int stages = fewest; stages <= kPairStages && s.best.cost >= 1e29; stages++) s.walk(n, kPairMaxRadix, stages + 1);
+    if (memo.size() < 4096) memo.emplace(key, s.best);
+    return s.best;
+}
+
+// Split of F into two passes of pair tiles: the divisor pair of the lowest
+// cost.  False when no pair of lengths has tiles.
+bool pair_split(int64_t F, std::vector<int> &out)
+{
+    double best = 1e29;
+    for (int64_t a = 2; a * a <= F; a++) {
+        if (F % a || F / a > kMaxPassRadix || F / a > 16 * a) continue;
+        const PairChoice x = pair_choice(static_cast<int>(F / a), false, true, F / a, 32);
+        const PairChoice y = pair_choice(static_cast<int>(a), false, false, a, 32);
+        if (x.cost + y.cost < best) {
+            best = x.cost + y.cost;
+            out = {static_cast<int>(F / a), static_cast<int>(a)};
+        }
+    }
+    return best < 1e29;
+}
+
 // Splits radices above max_r into supported pairs (16 = 4 x 4, 12 = 4 x 3);
 // false when a prime radix (11, 13) is above it.
 bool limit_radices(std::vector<int> &radices, int max_r)
@@ -266,6 +344,7 @@ struct Builder {
             s.db = false;
             s.db_fn = nullptr;
             s.cp_fn = nullptr;
+            s.pair = false;
             s.tc_fmt = -1;
             s.what += " [separated re/im]";
         }
@@ -294,7 +373,9 @@ struct Builder {
         int maxe_override = 0;
         int row_threads = p.row_threads;
         TuneChoice tc;
+        bool tuned = false;
         if (p.use_tuned && tuned_choice(n, tc) && valid_radices(tc.radices, n) && tc.maxe <= p.max_maxe) {
+            tuned = true;
             radices = tc.radices;
             maxe_override = tc.maxe;
             if (tc.row_threads > 0 && tc.row_threads <= p.row_threads) row_threads = tc.row_threads;
@@ -365,28 +446,172 @@ struct Builder {
                 }
                 s.grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(d.num_tiles, int64_t(per_sm) * sm_count(device))));
             }
-            // TMA column tiles of the same engine: box copies instead of per-element
-            // copies, last stage stored from registers
-            const void *cfn =
-                s.db_fn ? col_pipe_kernel_fn(n, d.tpt, d.tb, s.forward, d.out_a.estride == 1) : nullptr;
-            if (cfn && col_pipe_layout_ok(d)) {
-                const int64_t need = int64_t(d.tb) * std::max(n, d.pitch);
-                d.col_buf = (need + 15) / 16 * 16;
-                d.row_bufs = col_pipe_bufs(static_cast<int>(n), d.tpt, d.tb);
-                const int cps = kernel_blocks_per_sm(cfn, d.tb * d.tpt, col_pipe_smem(d));
-                if (cps > 0) {
-                    s.cp_fn = cfn;
-                    s.cp_grid = static_cast<int>(
-                        std::max<int64_t>(1, std::min<int64_t>(d.num_tiles, int64_t(cps) * sm_count(device))));
-                }
-            }
         }
+        if (column && io == IO_C2C && !add_column_variant(s)) return false;
+        if (!add_pair_variant(s, tuned ? &tc : nullptr)) return false;
         // passes of a multi-pass transform keep the FP32 kernels: their tiles would run on the
         // single-tile tensor-core kernel, several times slower than the double-buffered FP32 passes
         if (in_multipass || p.fft_type == 0x30 || !(io == IO_C2C || io == IO_R2C_PACKED || io == IO_C2R_PACKED))
             return true;
         const int form = tc_form(n);
         return form == 1 || form == 2 ? add_tc_variant(s, form) : true;
+    }
+
+    // TMA column tiles of two columns per thread where the length has an engine
+    // and the input fits its tensor map.  (The inter-pass twiddles of a
+    // multi-pass step are set by add_multipass.)
+    bool add_column_variant(Step &s)
+    {
+        ColPipe c;
+        if (!col_pipe_kernel(s.d.n, s.forward, s.d.out_a.estride == 1, c)) return true;
+        TileDesc d = s.d;
+        d.tb = c.tb;
+        d.tpt = c.tpt;
+        d.tiles_per_outer = (d.n_cols + d.tb - 1) / d.tb;
+        d.num_tiles = d.tiles_per_outer * d.n_outer;
+        d.nstages = c.nstages;
+        for (int i = 0; i < c.nstages; i++) d.radix[i] = c.radix[i];
+        if (!col_pipe_layout_ok(d)) return true;
+        TablePtr t = get_stage_table(c.radix, c.nstages, device, &err);
+        if (!t) return false;
+        p.tables.push_back(t);
+        d.stw = t->ptr;
+        d.dv_tiles = fast_div(d.tiles_per_outer);
+        d.dv_block = fast_div(d.out_a.cblock);
+        d.dv_gdiv = d.dv_gns = fast_div(1);
+        const int per_sm = kernel_blocks_per_sm(c.fn, d.tb / 2 * d.tpt, c.smem);
+        if (per_sm <= 0) return true;
+        s.cd = d;
+        s.cp_fn = c.fn;
+        s.cp_smem = c.smem;
+        s.cp_grid = static_cast<int>(
+            std::max<int64_t>(1, std::min<int64_t>(d.num_tiles, int64_t(per_sm) * sm_count(device))));
+        return true;
+    }
+
+    // columns of a pair tile of length n, 0 if it has none
+    static int pair_columns(int n) { return 2 * pair_choice(n, false, false, n, 32).P; }
+
+    // Pair tiles of a C2C column step, or of C2C / R2C / C2R rows without a
+    // compile-time engine, where the tile fits (pair_shape).
+    bool add_pair_variant(Step &s, const TuneChoice *tuned)
+    {
+        const TileDesc &d = s.d;
+        const bool rows = !d.xfast;
+        const int64_t most = int64_t(1) << 31;
+        if (d.n < 2 || d.n_cols >= most || d.n_outer >= most) return true;
+        int64_t in_dist = d.in_a.dist, out_dist = d.out_a.dist, max_pairs = 64;
+        if (rows) {
+            if (!(d.io == IO_C2C || d.io == IO_R2C_PACKED || d.io == IO_C2R_PACKED) || d.n_outer != 1 ||
+                d.in_a.estride != 1 || d.out_a.estride != 1 || (s.row_fn && !p.use_tuned))
+                return true;
+            in_dist = d.in_a.cstride;
+            out_dist = d.out_a.cstride;
+            // a tile of rows is copied as one run
+            if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
+        } else if (d.io != IO_C2C || d.in_a.cstride != 1 || d.in_a.cblock != 0 || d.out_a.cblock >= most) {
+            return true;
+        }
+        const bool runs = !rows && d.out_a.estride == 1;
+        // no more pairs than there are, and, in a launch of its own, fewer while there
+        // are too few tiles to occupy the SMs (columns keep eight pairs, 128-byte
+        // runs; a tile keeps 1024 points)
+        const int64_t pairs = d.n_outer * ((d.n_cols + 1) / 2);
+        while (max_pairs > 1 && max_pairs / 2 >= (d.n_cols + 1) / 2) max_pairs /= 2;
+        while (!p.use_tuned && max_pairs > (rows ? 1 : 8) && d.n * max_pairs > 1024 &&
+               pairs < max_pairs * sm_count(device) * 2)
+            max_pairs /= 2;
+        PairDesc q{};
+        std::vector<int> radices;
+        int P = static_cast<int>(max_pairs);
+        if (tuned) {
+            radices = tuned->radices;
+            if (tuned->row_threads > 0 && tuned->row_threads <= 128) P = std::min(P, 4);
+        } else {
+            const PairChoice c = pair_choice(d.n, rows, runs, in_dist, P);
+            radices = c.radices;
+            P = c.P;
+        }
+        while (P >= 1 && !pair_shape(q, d.n, radices.data(), static_cast<int>(radices.size()), rows, runs, in_dist, P)) P /= 2;
+        if (P < 1) return true;
+        const int64_t per_outer = (d.n_cols + 2 * q.P - 1) / (2 * q.P), tiles = per_outer * d.n_outer;
+        if (tiles >= most) return true;
+        const int per_sm = kernel_blocks_per_sm(pair_kernel_fn(s.forward), kPairThreads, pair_smem(q.buf_words));
+        if (per_sm <= 0) return true;
+        q.io = d.io;
+        q.n_cols = d.n_cols;
+        q.n_outer = d.n_outer;
+        q.tiles = static_cast<uint32_t>(tiles);
+        q.dv_tiles = fast_div(per_outer);
+        q.dv_block = fast_div(d.out_a.cblock);
+        q.dv_gdiv = q.dv_gns = fast_div(1);
+        q.dv_post = fast_div(d.n / 2 + 1);
+        q.in_a = d.in_a;
+        q.out_a = d.out_a;
+        if (rows) {
+            q.in_a = Addr{in_dist, in_dist, 1, 0, 0};
+            q.out_a = Addr{out_dist, out_dist, 1, 0, 0};
+        }
+        q.tw = d.tw;
+        if (q.nstages > 1) {
+            TablePtr t = get_stage_table(radices.data(), q.nstages, device, &err);
+            if (!t) return false;
+            p.tables.push_back(t);
+            q.stw = t->ptr;
+        }
+        s.pair = true;
+        s.pd = q;
+        s.pair_grid = static_cast<int>(std::min<int64_t>(tiles, int64_t(per_sm) * sm_count(device)));
+        return true;
+    }
+
+    // Inter-pass twiddle tables of a kernel of two columns per thread whose
+    // first radix is r0: t1 up to 8 MB (beyond it the rows of t1 come from the
+    // two-level table), t2 always.
+    bool pass_tables(const TileDesc &d, int r0, const float2 *&t1, const float2 *&t2)
+    {
+        const int64_t rows = d.n / r0;
+        if (rows * d.g_ns <= int64_t(1) << 20) {
+            TablePtr t = get_outer_table(rows, d.g_ns, d.g_ns * d.n, device, &err);
+            if (!t) return false;
+            p.tables.push_back(t);
+            t1 = t->ptr;
+        }
+        TablePtr t = get_outer_table(r0, d.g_ns, d.g_ns * r0, device, &err);
+        if (!t) return false;
+        p.tables.push_back(t);
+        t2 = t->ptr;
+        return true;
+    }
+
+    bool set_column_twiddles(Step &s)
+    {
+        const TileDesc &d = s.d;
+        if (s.cp_fn) {
+            TileDesc &c = s.cd;
+            c.g_twiddle = d.g_twiddle;
+            c.g_ns = d.g_ns;
+            c.g_div = d.g_div;
+            c.g_step = d.g_step;
+            c.g_lo = d.g_lo;
+            c.g_hi = d.g_hi;
+            c.g_log2l = d.g_log2l;
+            c.dv_gdiv = fast_div(d.g_div);
+            c.dv_gns = fast_div(d.g_ns);
+            if (d.g_twiddle && !pass_tables(d, c.radix[0], c.g_t1, c.g_t2)) return false;
+        }
+        if (s.pair) {
+            PairDesc &q = s.pd;
+            q.g_twiddle = d.g_twiddle;
+            q.g_step = d.g_step;
+            q.g_lo = d.g_lo;
+            q.g_hi = d.g_hi;
+            q.g_log2l = d.g_log2l;
+            q.dv_gdiv = fast_div(d.g_div);
+            q.dv_gns = fast_div(d.g_ns);
+            if (d.g_twiddle && !pass_tables(d, q.st[0].R, q.g_t1, q.g_t2)) return false;
+        }
+        return true;
     }
 
     // Stage arithmetic of a length-n step: 0 FP32, 1 FP16 x3, 2 BF16 x3 (in
@@ -589,9 +814,10 @@ struct Builder {
     bool add_multipass(int64_t F, int64_t outer, int64_t in_dist, int64_t out_dist, Buf src, Buf dst,
                        int64_t inner = 1)
     {
+        // powers of two: balanced passes on the compile-time engines
         std::vector<int> passes;
         int parts = 2;
-        while (!split_passes(F, parts, passes)) {
+        while (!((F & (F - 1)) != 0 && parts == 2 && pair_split(F, passes)) && !split_passes(F, parts, passes)) {
             if (++parts > 6) {
                 err = "length " + std::to_string(F) + " cannot be split into shared-memory passes";
                 return false;
@@ -630,6 +856,7 @@ struct Builder {
             d.g_lo = lo;
             d.g_hi = hi;
             d.g_log2l = log2l;
+            if (!set_column_twiddles(p.steps.back())) return false;
             ns *= rp;
             cur = nxt;
             cur_dist = nxt_dist;
@@ -808,23 +1035,19 @@ struct Builder {
             err = "strided axis of length " + std::to_string(n) + " has a prime factor above 13";
             return false;
         }
-        // Through transposes: the tensor-core form of lengths with the row pipeline,
-        // and FP32 axes above 1024 points without a TMA column engine, whose column
-        // tiles shrink to 2-4 columns (16-32-byte row runs).  Measured, 2D C2C
-        // (column axis strided; us, column kernel -> transposes): 4096^2 x 2
-        // 539 -> 391, 8192 x 1024 x 4 690 -> 419, 3000 x 1024 x 8 605 -> 454,
-        // 6561 x 512 x 8 548 -> 459, 1500^2 x 12 446 -> 345; 1000^2 x 64 1146 -> 1330
-        // and 2048^2 x 8 244 -> 374 (TMA column engine) stay on column tiles.
-        // Vertical 1D plans keep their column tiles (complex32 data converts in
-        // the first and last tile steps).
+        // Tensor-core forms of lengths with the row pipeline: through transposes.
+        // FP32 axes without a TMA column engine whose pair tile would keep at most
+        // four columns (32-byte row runs, lengths above about 512): as two passes of
+        // pair tiles, which keep 16 and more.  Vertical 1D plans keep their column
+        // tiles (complex32 data converts in the first and last tile steps).
         if (!in_multipass && p.fft_type != 0x30) {
             TcConfig tcc;
             const int form = tc_form(n);
-            const bool tc = (form == 1 || form == 2) && tc_rows_config(static_cast<int>(n), tcc);
-            const bool slow_columns =
-                form == 0 && !p.vertical && n > 1024 && n <= kMaxStridedTile &&
-                !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0);
-            if (tc || slow_columns) return add_transposed_axis(n, outer, inner, src, dst);
+            if ((form == 1 || form == 2) && tc_rows_config(static_cast<int>(n), tcc))
+                return add_transposed_axis(n, outer, inner, src, dst);
+            if (form == 0 && !p.vertical && n > 256 && n <= kMaxStridedTile && inner > 1 &&
+                !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
+                return add_multipass(n, outer, n * inner, n * inner, src, dst, inner);
         }
         TileCfg c;
         if (n > kMaxStridedTile || !choose_cfg(static_cast<int>(n), true, inner, c, err)) {
@@ -1137,6 +1360,13 @@ std::string describe_plan(const Plan &p)
     for (const Step &s : p.steps) {
         o << "  [" << static_cast<int>(s.src) << "->" << static_cast<int>(s.dst) << "] " << s.what;
         if (s.kind == StepKind::kTile) {
+            if (s.pair && !s.cp_fn && !s.row_fn && s.tc_fmt < 0) {
+                o << " [pair tiles] n=" << s.pd.n << " radices=";
+                for (int i = 0; i < s.pd.nstages; i++) o << (i ? "x" : "") << s.pd.st[i].R;
+                o << " pairs=" << s.pd.P << " tiles=" << s.pd.tiles << " grid=" << s.pair_grid
+                  << " smem=" << pair_smem(s.pd.buf_words) << "\n";
+                continue;
+            }
             o << (s.cp_fn ? " [TMA column tiles, static engine]"
                           : (s.db ? (s.db_fn ? " [double-buffered, static engine]" : " [double-buffered]") : ""))
               << " n=" << s.d.n

@@ -87,6 +87,31 @@ TablePtr get_stage_table(const int *radix, int nstages, int device, std::string 
     return t;
 }
 
+TablePtr get_outer_table(int64_t rows, int64_t ns, int64_t denom, int device, std::string *err)
+{
+    static std::mutex mu;
+    static std::map<std::tuple<int, int64_t, int64_t, int64_t>, std::weak_ptr<DeviceTable>> cache;
+    std::lock_guard<std::mutex> lock(mu);
+    auto key = std::make_tuple(device, rows, ns, denom);
+    auto it = cache.find(key);
+    if (it != cache.end()) {
+        if (TablePtr t = it->second.lock()) return t;
+    }
+    auto t = std::make_shared<DeviceTable>();
+    t->count = rows * ns;
+    t->device = device;
+    cudaError_t e = cudaMalloc(&t->ptr, sizeof(float2) * static_cast<size_t>(t->count));
+    if (e == cudaSuccess) e = fill_outer_twiddles(t->ptr, rows, ns, denom, 0);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    if (e != cudaSuccess) {
+        if (err) *err = std::string("twiddle table: ") + cudaGetErrorString(e);
+        cudaGetLastError();
+        return nullptr;
+    }
+    cache[key] = t;
+    return t;
+}
+
 TablePtr get_tc_matrix(int N, int fmt, bool fwd, int device, std::string *err, int layout)
 {
     static std::mutex mu;
@@ -160,6 +185,7 @@ cudaError_t configure_kernels(int device)
     tc_kernel_fns(fns);
     tc_rows_kernel_fns(fns);
     col_pipe_kernel_fns(fns);
+    pair_kernel_fns(fns);
     for (const void *fn : fns) {
         cudaError_t e = allow_max_dynamic_smem(fn);
         if (e != cudaSuccess) return e;
@@ -206,6 +232,7 @@ std::string complex32_steps(const Plan &p, std::vector<Step> &out)
         s->db = false;
         s->db_fn = nullptr;
         s->cp_fn = nullptr;
+        s->pair = false;
     }
     out.front().d.half_io |= 1;
     out.back().d.half_io |= 2;
@@ -235,6 +262,23 @@ bool scale_steps_to_rows(const Plan &p, int64_t rows, std::vector<Step> &out)
             return false;
         }
         s.grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(d.num_tiles, s.grid)));
+        if (s.pair) {
+            PairDesc &q = s.pd;
+            if (q.rows) {
+                q.n_cols = rows;
+                q.tiles = static_cast<uint32_t>((rows + 2 * q.P - 1) / (2 * q.P));
+            } else {
+                q.n_outer = rows;
+                q.tiles = static_cast<uint32_t>(q.dv_tiles.d * rows);
+            }
+            s.pair_grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(q.tiles, s.pair_grid)));
+        }
+        if (s.cp_fn) {
+            // multi-pass step on the column kernel: one outer group per transform
+            s.cd.n_outer = rows;
+            s.cd.num_tiles = s.cd.tiles_per_outer * rows;
+            s.cp_grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(s.cd.num_tiles, s.cp_grid)));
+        }
         if (s.has_row) {
             TileDesc &r = s.rd;
             r.n_cols = rows;
@@ -278,6 +322,11 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                     d.out = dst;
                     e = launch_tc(d, d.n, s.tc_fmt, s.forward, s.tc_mat, s.tc_tw, s.grid, device_error_word(p.device),
                                   st);
+                } else if (s.pair && !s.cp_fn && !s.row_fn && (!s.pd.rows || src != dst)) {
+                    PairDesc d = s.pd;
+                    d.in = src;
+                    d.out = dst;
+                    e = launch_pair(d, s.forward, s.pair_grid, st);
                 } else if (s.has_row && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && src != dst) {
                     TileDesc d = s.rd;
                     d.in = src;
@@ -288,11 +337,16 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                     else
                         e = launch_row_tiles(d, s.maxe, s.forward, s.row_grid, device_error_word(p.device), st);
                 } else if (s.cp_fn && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-                    TileDesc d = s.d;
+                    TileDesc d = s.cd;
                     d.in = src;
                     d.out = dst;
-                    d.stw = s.db_stw;
-                    e = launch_col_pipe(s.cp_fn, d, s.cp_grid, device_error_word(p.device), st);
+                    e = launch_col_pipe(s.cp_fn, d, s.cp_smem, s.cp_grid, device_error_word(p.device), st);
+                } else if (s.pair && (!s.pd.rows || src != dst)) {
+                    // a source that the static engines' bulk copies cannot read
+                    PairDesc d = s.pd;
+                    d.in = src;
+                    d.out = dst;
+                    e = launch_pair(d, s.forward, s.pair_grid, st);
                 } else if (s.db) {
                     TileDesc d = s.d;
                     d.in = src;

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "fft_tile.cuh"
+#include "pair_tile.cuh"
 
 namespace sipfft {
 
@@ -48,6 +49,7 @@ void static_kernel_fns(std::vector<const void *> &out);
 constexpr int kBatchBlock = 256;
 constexpr int kBatchMaxe = 16;
 constexpr int64_t kBatchMaxRowN = 4096;
+constexpr int64_t kPairMaxRowN = 2048;  // the same for batches on the pair kernel
 const void *batch_kernel_fn(bool forward, bool compact);
 cudaError_t launch_batch(int grid, int block, size_t smem, const BatchSeg *segs, const int2 *items, int nitems,
                          int *counter, int *done, const BatchBufs &bufs, int *err, bool forward, bool compact,
@@ -69,19 +71,32 @@ struct StaticKernel {
     int row_bufs = 2;           // shared-memory buffers of its row kernel (3: ping-pong work area)
 };
 const StaticKernel *find_static_kernel(int n, int io);
-// TMA-pipelined column kernels (col_pipe.cu) for the power-of-two static
-// engines with 16 points per thread: n, threads per transform and columns per
-// tile must match an instantiation.  contiguous_out: each column's outputs are
-// contiguous (output element stride 1); the variant that stages them through
-// shared memory is returned where one exists.
-const void *col_pipe_kernel_fn(int n, int tpt, int tb, bool forward, bool contiguous_out);
+// TMA-pipelined column kernels (col_pipe.cu): the engine of a length, its
+// threads per pair of columns, columns per tile and shared memory.
+// contiguous_out: each column's outputs are contiguous (element stride 1); the
+// variant that stores whole runs of a column is returned where one exists.
+struct ColPipe {
+    const void *fn = nullptr;
+    int tpt = 0, tb = 0;
+    size_t smem = 0;
+    int nstages = 0, radix[4] = {};
+};
+bool col_pipe_kernel(int n, bool forward, bool contiguous_out, ColPipe &c);
 bool col_pipe_has_engine(int n);  // a TMA column engine exists for this length
-int col_pipe_bufs(int n, int tpt, int tb);  // its shared-memory tile buffers (TileDesc::row_bufs)
 void col_pipe_kernel_fns(std::vector<const void *> &out);
-size_t col_pipe_smem(const TileDesc &d);
 // the step's input addressing and sizes fit the tensor map of the column kernel
 bool col_pipe_layout_ok(const TileDesc &d);
-cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, int grid, int *err, cudaStream_t st);
+cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, size_t smem, int grid, int *err, cudaStream_t st);
+// Runtime-radix tiles of two rows or columns per thread (pair_tile_impl.cuh).
+const void *pair_kernel_fn(bool forward);
+const void *pair_batch_fn(bool forward);
+void pair_kernel_fns(std::vector<const void *> &out);
+size_t pair_smem(int buf_words);
+cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st);
+cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems, int *counter,
+                              int *done, const BatchBufs &bufs, int *err, bool forward, cudaStream_t st);
+// t[j * ns + k] = exp(-2 pi i j k / denom), j < rows, k < ns
+cudaError_t fill_outer_twiddles(float2 *t, int64_t rows, int64_t ns, int64_t denom, cudaStream_t st);
 cudaError_t fill_stage_twiddles(float2 *t, const int *radix, int nstages, cudaStream_t st);
 int64_t stage_twiddle_count(const int *radix, int nstages);
 // Tensor-core split-precision stages (tc_fft.cu): n = n1 * n2 as two DFT-matrix
@@ -154,6 +169,8 @@ TablePtr get_stage_table(const StaticKernel &k, int device, std::string *err);
 // per-stage twiddle tables of any radix sequence: stage s >= 1 holds
 // W_{ns R}^{r k} at [(r-1) ns + k], stages back to back (stage 0 has none)
 TablePtr get_stage_table(const int *radix, int nstages, int device, std::string *err);
+// exp(-2 pi i j k / denom) at [j * ns + k], j < rows, k < ns
+TablePtr get_outer_table(int64_t rows, int64_t ns, int64_t denom, int device, std::string *err);
 // hi/lo operand matrices of one tensor-core stage (N points, fmt, direction).
 // layout 0 (A operand of tc_fft_kernel): hi at ptr, lo at ptr + 64 N float2,
 // each 128 x 2N 16-bit values; layout 1 (B operand of tc_rows_kernel): hi at
@@ -190,6 +207,12 @@ struct Step {
     // TMA column kernel of the same engine (used when the source is 16-byte aligned)
     const void *cp_fn = nullptr;
     int cp_grid = 1;
+    size_t cp_smem = 0;
+    TileDesc cd{};
+    // runtime-radix pair tiles (no alignment requirement)
+    bool pair = false;
+    PairDesc pd{};
+    int pair_grid = 1;
     bool has_row = false;
     TileDesc rd{};
     int row_grid = 1;

@@ -88,7 +88,7 @@ constexpr int static_maxv()
 // half-length table a CTA keeps in L1 shrink to NBF entries (used from 2048
 // points, where the whole table no longer fits next to the stage tables).
 template <class Src>
-__device__ __forceinline__ float2 fetch(const Src &src, int j, int off)
+__device__ __forceinline__ auto fetch(const Src &src, int j, int off)
 {
     return src(j + off);
 }
@@ -98,8 +98,8 @@ __device__ __forceinline__ float2 fetch(const C2RPre<FWD> &src, int j, int off)
     return src.split(j, off);
 }
 
-template <class Q, int S, int T, bool FWD, class Src>
-__device__ __forceinline__ void sgather(float2 *v, const Src &src, int lane, bool active,
+template <class Q, int S, int T, bool FWD, class V, class Src>
+__device__ __forceinline__ void sgather(V *v, const Src &src, int lane, bool active,
                                         const float2 *__restrict__ stw)
 {
     constexpr int R = Q::r[S], N = Q::N, NS = Q::ns(S), NBF = N / R, NB = (NBF + T - 1) / T;
@@ -152,8 +152,8 @@ __device__ __forceinline__ void sgather(float2 *v, const Src &src, int lane, boo
     }
 }
 
-template <class Q, int S, int T, class Dst>
-__device__ __forceinline__ void sscatter(const float2 *v, const Dst &dst, int lane, bool active)
+template <class Q, int S, int T, class V, class Dst>
+__device__ __forceinline__ void sscatter(const V *v, const Dst &dst, int lane, bool active)
 {
     constexpr int R = Q::r[S], N = Q::N, NS = Q::ns(S), NBF = N / R, NB = (NBF + T - 1) / T;
 #pragma unroll

@@ -23,6 +23,14 @@ __device__ __forceinline__ int64_t col_base(const Addr &a, int64_t o, int64_t c)
     return x;
 }
 
+// the same with 32-bit column arithmetic; block: the divisor of a.cblock
+__device__ __forceinline__ int64_t col_base32(const Addr &a, const FastDiv &block, uint32_t o, uint32_t c)
+{
+    int64_t x = o * a.dist + c * a.cstride;
+    if (a.cblock) x += block.div(c) * a.cjump;
+    return x;
+}
+
 // W_F^(e kc step) from the two-level table.  The exponent is below F (e < n,
 // kc < Ns, step = F / (Ns n)), and every multi-pass length F is at most 2^28
 // (transforms up to 2^27 points, Bluestein convolutions up to 2^28), so the
