@@ -293,6 +293,7 @@ std::string build_batch_with(BatchPlan &bp)
         p.row_threads = 256;
         p.row_smem = 48 * 1024;
         p.max_row_n = bp.pairs ? kPairMaxRowN : kBatchMaxRowN;
+        p.pair_buf = bp.pairs ? kPairBufBytes4 : 0;
         p.max_maxe = kBatchMaxe;
         p.max_radix = bp.compact ? kCompactMaxRadix : 16;
         std::string e = build_plan_1d(p);
@@ -328,6 +329,10 @@ std::string build_batch_with(BatchPlan &bp)
                 ps.in_buf = sg.in_buf;
                 ps.out_buf = sg.out_buf;
                 ps.dep = sg.dep;
+                if (sg.dep >= 0) {
+                    ps.dep_tiles = static_cast<int>(bp.pair_segs[sg.dep].d.tiles);
+                    bp.pair_segs[sg.dep].consumed = 1;
+                }
                 bp.pair_segs.push_back(ps);
                 bp.buf_words = std::max(bp.buf_words, s.pd.buf_words);
                 const int phase = p.steps.size() == 1 ? 1 : (i == 0 ? 0 : static_cast<int>(i) + 1);
@@ -419,7 +424,7 @@ cudaError_t enqueue(BatchPlan &bp, const void *in, void *out, void *ws, cudaStre
     BatchBufs bufs{{const_cast<void *>(in), out, ws, nullptr}};
     if (bp.pairs)
         return launch_pair_batch(bp.grid, bp.buf_words, bp.d_pair_segs, bp.d_items, static_cast<int>(bp.items.size()),
-                                 bp.d_counters, bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, st);
+                                 bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, st);
     return launch_batch(bp.grid, bp.block, bp.smem, bp.d_segs, bp.d_items, static_cast<int>(bp.items.size()),
                         bp.d_counters, bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, bp.compact,
                         st);

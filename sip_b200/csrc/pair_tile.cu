@@ -25,7 +25,7 @@ void pair_kernel_fns(std::vector<const void *> &out)
 
 size_t pair_smem(int buf_words)
 {
-    const size_t head = ((2 * ((sizeof(PairSeg) + 15) / 16)) + 7) / 8 * 8;
+    const size_t head = ((kPairSlots * ((sizeof(PairSeg) + 15) / 16)) + 7) / 8 * 8;
     return (head + size_t(2) * buf_words) * 16;
 }
 
@@ -39,11 +39,11 @@ cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t 
     return launch_pdl(pair_kernel_fn(forward), dim3(grid), dim3(kPairThreads), smem, st, args);
 }
 
-cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems, int *counter,
+cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,
                               int *done, const BatchBufs &bufs, int *err, bool forward, cudaStream_t st)
 {
     BatchBufs b = bufs;
-    void *args[] = {&segs, &items, &nitems, &counter, &done, &b, &err, &buf_words};
+    void *args[] = {&segs, &items, &nitems, &done, &b, &err, &buf_words};
     return cudaLaunchKernel(pair_batch_fn(forward), dim3(grid), dim3(kPairThreads), args, pair_smem(buf_words), st);
 }
 

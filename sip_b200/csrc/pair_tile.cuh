@@ -8,6 +8,8 @@
 namespace sipfft {
 
 constexpr int kPairThreads = 128;   // threads per CTA
+constexpr int kPairSlots = 3;       // descriptors in shared memory
+constexpr int kPairKnown = 2048;    // producers of an uneven batch that a CTA remembers as finished
 constexpr int kPairStages = 8;      // most stages of a tile
 constexpr int kPairMaxRadix = 16;   // radices 2..16
 constexpr int kPairBufBytes = 37504;  // most shared memory of one tile buffer (two per CTA, three CTAs per SM)
@@ -46,6 +48,10 @@ struct PairDesc {
     uint32_t tiles;
     FastDiv dv_tiles, dv_block, dv_gdiv, dv_gns, dv_post;
     Addr in_a, out_a;  // rows: row distances in in_a.dist / out_a.dist
+    // 32-bit copies of the strides that the stages use, and the distance of the
+    // odd column of a pair from the even one (-1: crosses column blocks, computed)
+    uint32_t in_es, out_es, out_cs;
+    int32_t out_jump, out_delta;
     const float2 *stw;  // per-stage twiddle tables
     const float2 *tw;   // exp(-2 pi i k / 2n) of the packed real kinds
     int g_twiddle;
@@ -55,24 +61,26 @@ struct PairDesc {
 };
 
 // One segment of an uneven batch on the pair kernel (offsets in bytes into
-// the buffers of BatchBufs; dep: the segment whose output this one reads).
+// the buffers of BatchBufs; dep: the segment whose output this one reads and
+// its tile count; consumed: another segment reads this one's output).
 struct alignas(16) PairSeg {
     PairDesc d;
     int64_t in_off, out_off;
     int in_buf, out_buf;
-    int dep, pad_;
+    int dep, dep_tiles, consumed;
 };
 
 // Relative cost per point of a tile of P pairs: every thread runs every
 // butterfly slot of a stage (about eight instructions of addressing,
 // shared-memory and twiddle work per point and the butterfly's FP32 operations,
-// halved by packing), a tile costs about 260 instructions a thread besides, and
-// columns in row runs below 128 bytes waste memory transactions.
+// halved by packing; about 24 per butterfly for its indices), a tile costs about
+// 350 instructions a thread besides, and columns in row runs below 128 bytes
+// waste memory transactions.
 inline double pair_tile_cost(int n, const int *radix, int nstages, bool rows, int P, int buf_words)
 {
     static const double flops[] = {0, 0, 2, 5.3, 4, 7.2, 7.3, 11, 6.5, 11.5, 9.2, 18, 9.3, 22, 13, 12.5, 9.3};
-    double c = 260.0;
-    for (int s = 0; s < nstages; s++) c += pair_nb(radix[s]) * radix[s] * (8.0 + flops[radix[s]]);
+    double c = 350.0;
+    for (int s = 0; s < nstages; s++) c += pair_nb(radix[s]) * (24.0 + radix[s] * (8.0 + flops[radix[s]]));
     c *= double(kPairThreads) / (double(n) * P);
     if (buf_words * 16 > kPairBufBytes4) c *= 1.12;
     if (!rows) c *= P >= 8 ? 1.0 : (P == 4 ? 1.15 : (P == 2 ? 1.6 : 2.5));
@@ -82,7 +90,8 @@ inline double pair_tile_cost(int n, const int *radix, int nstages, bool rows, in
 // Tile shape for a transform of length n with these radices and P pairs per
 // tile (columns: a power of two): every stage must fit the threads' butterflies
 // and the staged rows (raw_dist elements apart; columns: n) a tile buffer.
-inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool rows, bool runs, int64_t raw_dist, int P)
+inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool rows, bool runs, int64_t raw_dist, int P,
+                       int max_buf = kPairBufBytes)
 {
     if (n < 2 || nstages < 1 || nstages > kPairStages || P < 1 || P > kPairThreads) return false;
     d.n = n;
@@ -106,7 +115,7 @@ inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool r
     const int64_t work = rows ? int64_t(P - 1) * d.SP + elems : int64_t(elems - 1) * d.SE + P;
     const int64_t raw = rows ? (2 * P * raw_dist + 3) / 2 : int64_t(n) * P;
     const int64_t words = ((work > raw ? work : raw) + 7) / 8 * 8;
-    if (words * 16 > kPairBufBytes) return false;
+    if (words * 16 > max_buf) return false;
     d.buf_words = static_cast<int>(words);
     int ns = 1, toff = 0;
     for (int s = 0; s < nstages; s++) {
@@ -129,13 +138,13 @@ inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool r
 
 // Work-tile words of butterfly (p, j) of stage t: its first input (the others
 // follow t.gstep apart) and its first output (ns * SE apart).
-__host__ __device__ __forceinline__ int pair_gather_at(const PairDesc &d, const PairStage &t, int p, int j, int q)
+__host__ __device__ __forceinline__ int pair_gather_at(int SP, int SE, int gpad, int p, int j, int q)
 {
-    return p * d.SP + (j + (t.gpad ? q : 0)) * d.SE;  // q = j div ns
+    return p * SP + (j + (gpad ? q : 0)) * SE;  // q = j div ns
 }
-__host__ __device__ __forceinline__ int pair_scatter_at(const PairDesc &d, const PairStage &t, int p, int j, int q)
+__host__ __device__ __forceinline__ int pair_scatter_at(int SP, int SE, int spad, int ns, int R, int p, int j, int q)
 {
-    return p * d.SP + (j + q * t.ns * (t.R - 1) + (t.spad ? j : 0)) * d.SE;  // q ns R + (j - q ns)
+    return p * SP + (j + q * ns * (R - 1) + (spad ? j : 0)) * SE;  // q ns R + (j - q ns)
 }
 
 }  // namespace sipfft

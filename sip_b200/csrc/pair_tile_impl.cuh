@@ -32,6 +32,8 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------------ tile copies
 // Rows: the tile is one run of elements; it lands one element in when its
 // first element is not 16-byte aligned, so that the rest copies in 16-byte
@@ -52,6 +54,7 @@ __device__ __forceinline__ void pair_issue(const PairDesc &d, const void *in, fl
         float2 *dst = reinterpret_cast<float2 *>(buf) + mis;
         if (mis && tid == 0) cp_async8(dst, src);
         const int chunks = (count - mis) >> 1;
+#pragma unroll 4
         for (int i = tid; i < chunks; i += kPairThreads) cp_async16(dst + mis + 2 * i, src + mis + 2 * i);
         if (((count - mis) & 1) && tid == 0) cp_async8(dst + count - 1, src + count - 1);
         return;
@@ -60,15 +63,17 @@ __device__ __forceinline__ void pair_issue(const PairDesc &d, const void *in, fl
     const int p = tid & (d.P - 1);
     const int64_t c = int64_t(t - o * d.dv_tiles.d) * (2 * d.P) + 2 * p;
     if (c >= d.n_cols) return;
-    const int64_t es = d.in_a.estride;
-    const float2 *src = x + o * d.in_a.dist + c + (tid >> d.lp) * es;
+    const uint32_t es = d.in_es;
+    const float2 *src = x + o * d.in_a.dist + c + static_cast<uint64_t>(static_cast<uint32_t>(tid) >> d.lp) * es;
     float4 *dst = buf + tid;
-    const int64_t step = (kPairThreads >> d.lp) * es;
+    const uint64_t step = static_cast<uint64_t>(kPairThreads >> d.lp) * es;
     const int total = d.n * d.P;
     if (c + 1 < d.n_cols) {
         if (((reinterpret_cast<uintptr_t>(src) & 15) == 0) && es % 2 == 0) {
+#pragma unroll 4
             for (int i = tid; i < total; i += kPairThreads, dst += kPairThreads, src += step) cp_async16(dst, src);
         } else {
+#pragma unroll 4
             for (int i = tid; i < total; i += kPairThreads, dst += kPairThreads, src += step) {
                 cp_async8(dst, src);
                 cp_async8(reinterpret_cast<float2 *>(dst) + 1, src + 1);
@@ -80,10 +85,10 @@ __device__ __forceinline__ void pair_issue(const PairDesc &d, const void *in, fl
 }
 
 // ------------------------------------------------------------------------------------ stages
-// A CTA's shared memory: two slots for the segments (descriptors) of the tile
-// being transformed and of the next one, then the two tile buffers.
+// A CTA's shared memory: slots for the segments (descriptors) of the tile
+// being transformed and of the next two, then the two tile buffers.
 constexpr int kPairSlotWords = (sizeof(PairSeg) + 15) / 16;
-constexpr int kPairHeadWords = (2 * kPairSlotWords + 7) / 8 * 8;
+constexpr int kPairHeadWords = (kPairSlots * kPairSlotWords + 7) / 8 * 8;
 
 extern __shared__ __align__(128) float4 pair_smem[];
 
@@ -97,15 +102,18 @@ struct PairTileState {
     int slot;           // descriptor
     int buf;            // first word of the tile buffer
     int mis;            // rows: elements that the staged rows start into the buffer
-    float2 *out;
-    uint32_t o, c0;     // outer index and first column (rows: first row) of the tile
+    float2 *out;        // outputs of the tile's outer index
+    uint32_t c0;        // first column (rows: first row) of the tile
     uint32_t left;      // columns (rows) from c0 on
 };
 
 __device__ __forceinline__ cpx2 word_in(float4 q) { return {make_float2(q.x, q.y), make_float2(q.z, q.w)}; }
 __device__ __forceinline__ float4 word_of(cpx2 v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
 
-enum PairSource { kPairWork = 0, kPairRows = 1, kPairCols = 2, kPairColsTwiddled = 3 };
+// Where a stage reads, and how the threads walk the tile: rows with the
+// elements fastest, columns with the pairs fastest; a work tile either way (the
+// last stage of columns whose outputs are contiguous takes the elements fastest).
+enum PairSource { kPairRows = 0, kPairCols = 1, kPairColsTwiddled = 2, kPairWorkE = 3, kPairWorkP = 4 };
 
 // One stage of radix R: reads the staged tile (rows, columns, columns with the
 // inter-pass twiddles of a multi-pass step) or the work tile, writes the work
@@ -116,32 +124,45 @@ template <int R, PairSource SRC, bool FWD>
 __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTileState s)
 {
     constexpr int NB = pair_nb(R);
-    constexpr bool FIRST = SRC != kPairWork;
+    constexpr bool FIRST = SRC <= kPairColsTwiddled;
+    constexpr bool E = SRC == kPairRows || SRC == kPairWorkE;  // elements fastest
     const PairDesc &d = pair_slot(s.slot).d;
     const PairStage &t = d.st[stage];
-    const int nbf = t.nbf, tasks = t.tasks, ns = FIRST ? 1 : t.ns, lp = d.lp;
-    const bool fast_e = SRC == kPairRows || d.rows || (to_global && d.runs);  // elements fastest
-    const uint32_t nbf_m = t.nbf_m, ns_m = t.ns_m;
+    const int tid = static_cast<int>(threadIdx.x);
+    // (copied out of shared memory once: stores and barriers would reload them)
+    const int nbf = t.nbf, ns = FIRST ? 1 : t.ns, lp = d.lp, tasks = t.tasks, SP = d.SP, SE = d.SE, spad = t.spad;
+    const uint32_t ns_m = t.ns_m, nbf_m = t.nbf_m;
     cpx2 v[NB * R];
-    // butterfly b of this thread: pair p, index j, block q = j div ns
-    auto task = [&](int b, int &p, int &j, int &q) {
-        int i = static_cast<int>(threadIdx.x) + b * kPairThreads;
-        const bool on = i < tasks;
-        i = on ? i : 0;
-        if (fast_e) {
-            p = nbf == 1 ? i : static_cast<int>(__umulhi(static_cast<uint32_t>(i), nbf_m));
-            j = i - p * nbf;
+    // butterfly b of this thread: pair p, index j; false beyond the tile
+    const int p0 = tid & ((1 << lp) - 1), j0 = tid >> lp, dj = kPairThreads >> lp;
+    auto task = [&](int b, int &p, int &j) -> bool {
+        if constexpr (E) {
+            const int i = tid + b * kPairThreads;
+            const bool on = i < tasks;
+            const int u = on ? i : 0;
+            p = nbf == 1 ? u : static_cast<int>(__umulhi(static_cast<uint32_t>(u), nbf_m));
+            j = u - p * nbf;
+            return on;
         } else {
-            p = i & ((1 << lp) - 1);
-            j = i >> lp;
+            p = p0;
+            j = j0 + b * dj;
+            const bool on = j < nbf;
+            j = on ? j : 0;
+            return on;
         }
-        q = FIRST ? j : static_cast<int>(__umulhi(static_cast<uint32_t>(j), ns_m));
-        return on;
     };
+    auto block = [&](int j) { return FIRST ? j : static_cast<int>(__umulhi(static_cast<uint32_t>(j), ns_m)); };  // j div ns
+    PassTwiddle tw{};
+    PassTable2 two{};
+    if constexpr (SRC == kPairColsTwiddled) {
+        const uint32_t c = s.c0 + 2 * p0;
+        tw = PassTwiddle{d.g_t1, d.g_t2, d.dv_gns.d, d.dv_gns.mod(d.dv_gdiv.div(c)), d.dv_gns.mod(d.dv_gdiv.div(c + 1))};
+        two = PassTable2{d.g_lo, d.g_hi, d.g_log2l, static_cast<uint32_t>(d.g_step)};
+    }
 #pragma unroll
     for (int b = 0; b < NB; b++) {
-        int p, j, q;
-        task(b, p, j, q);
+        int p, j;
+        task(b, p, j);
         if constexpr (SRC == kPairRows) {
             const int dist = static_cast<int>(d.in_a.dist);
             const float2 *x0 = reinterpret_cast<const float2 *>(pair_smem + s.buf) + s.mis + (2 * p) * dist + j;
@@ -156,38 +177,46 @@ __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTil
                 const float4 u = w[r * step];
                 v[b * R + r] = pair_of(make_float2(u.x, u.y), make_float2(u.z, u.w));
             }
-            if constexpr (SRC == kPairColsTwiddled) {
-                const uint32_t c = s.c0 + 2 * p;
-                const PassTwiddle tw{d.g_t1, d.g_t2, d.dv_gns.d, d.dv_gns.mod(d.dv_gdiv.div(c)),
-                                     d.dv_gns.mod(d.dv_gdiv.div(c + 1))};
-                const PassTable2 two{d.g_lo, d.g_hi, d.g_log2l, static_cast<uint32_t>(d.g_step)};
-                tw.template apply<R, FWD, false>(v + b * R, j, two);
-            }
+            if constexpr (SRC == kPairColsTwiddled) tw.template apply<R, FWD, false>(v + b * R, j, two);
         } else {
-            const float4 *w = pair_smem + s.buf + pair_gather_at(d, t, p, j, q);
+            const int q = block(j);
+            const float4 *w = pair_smem + s.buf + pair_gather_at(SP, SE, t.gpad, p, j, q);
             const int step = t.gstep;
 #pragma unroll
             for (int r = 0; r < R; r++) v[b * R + r] = word_in(w[r * step]);
-            const float2 *tw = d.stw + t.toff + (j - q * ns);
+            const float2 *wt = d.stw + t.toff + (j - q * ns);
 #pragma unroll
-            for (int r = 1; r < R; r++) v[b * R + r] = cmul(v[b * R + r], dir<FWD>(__ldg(tw + (r - 1) * ns)));
+            for (int r = 1; r < R; r++) v[b * R + r] = cmul(v[b * R + r], dir<FWD>(__ldg(wt + (r - 1) * ns)));
         }
         dft<R, FWD>(v + b * R);
     }
     if (to_global) {
-        const int64_t es = d.out_a.estride, step = ns * es;
+        const uint32_t es = d.out_es;
+        const uint64_t step = static_cast<uint64_t>(static_cast<uint32_t>(ns)) * es;
+        const int delta0 = d.out_delta, jump = d.out_jump;
+        const uint32_t cs = d.out_cs;
+        const FastDiv by_block = d.dv_block;
+        // first element of the even column of pair p, and the odd column's distance
+        auto column = [&](int p, int64_t &delta) -> float2 * {
+            const uint32_t c = s.c0 + 2 * p;
+            const uint32_t blk = jump ? by_block.div(c) : 0u;
+            delta = delta0 >= 0 ? delta0 : int64_t(cs) + int64_t(by_block.div(c + 1) - blk) * jump;
+            return s.out + (static_cast<uint64_t>(c) * cs + static_cast<uint64_t>(blk) * static_cast<uint32_t>(jump));
+        };
+        int64_t delta = 0;
+        float2 *base = E ? nullptr : column(p0, delta);
 #pragma unroll
         for (int b = 0; b < NB; b++) {
-            int p, j, q;
-            if (task(b, p, j, q) && static_cast<uint32_t>(2 * p) < s.left) {
-                const uint32_t c = s.c0 + 2 * p;
+            int p, j;
+            if (task(b, p, j) && static_cast<uint32_t>(2 * p) < s.left) {
+                if constexpr (E) base = column(p, delta);
+                float2 *y0 = base + static_cast<uint64_t>(static_cast<uint32_t>(j)) * es;
                 const bool second = static_cast<uint32_t>(2 * p + 1) < s.left;
-                float2 *y0 = s.out + col_base32(d.out_a, d.dv_block, s.o, c) + j * es;
-                float2 *y1 = s.out + col_base32(d.out_a, d.dv_block, s.o, c + 1) + j * es;
-                if (second && y1 == y0 + 1 && ((reinterpret_cast<uintptr_t>(y0) & 15) == 0) && es % 2 == 0) {
+                if (!E && second && delta == 1 && ((reinterpret_cast<uintptr_t>(y0) & 15) == 0) && es % 2 == 0) {
 #pragma unroll
                     for (int r = 0; r < R; r++, y0 += step) st_stream(y0, first_of(v[b * R + r]), second_of(v[b * R + r]));
                 } else {
+                    float2 *y1 = y0 + delta;
 #pragma unroll
                     for (int r = 0; r < R; r++, y0 += step) st_stream(y0, first_of(v[b * R + r]));
                     if (second) {
@@ -202,10 +231,10 @@ __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTil
     __syncthreads();
 #pragma unroll
     for (int b = 0; b < NB; b++) {
-        int p, j, q;
-        if (task(b, p, j, q)) {
-            float4 *w = pair_smem + s.buf + pair_scatter_at(d, t, p, j, q);
-            const int step = ns * d.SE;
+        int p, j;
+        if (task(b, p, j)) {
+            float4 *w = pair_smem + s.buf + pair_scatter_at(SP, SE, spad, ns, R, p, j, block(j));
+            const int step = ns * SE;
 #pragma unroll
             for (int r = 0; r < R; r++) w[r * step] = word_of(v[b * R + r]);
         }
@@ -292,15 +321,15 @@ __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, voi
     PairTileState s;
     s.slot = slot;
     s.buf = buf;
-    s.out = static_cast<float2 *>(out);
     s.mis = 0;
     if (d.rows) {
+        s.out = static_cast<float2 *>(out);
         s.mis = static_cast<int>((reinterpret_cast<uintptr_t>(static_cast<const float2 *>(in) + pair_row_start(d, t)) >> 3) & 1);
-        s.o = 0;
         s.c0 = t * (2 * d.P);
     } else {
-        s.o = d.dv_tiles.div(t);
-        s.c0 = (t - s.o * d.dv_tiles.d) * (2 * d.P);
+        const uint32_t o = d.dv_tiles.div(t);
+        s.c0 = (t - o * d.dv_tiles.d) * (2 * d.P);
+        s.out = static_cast<float2 *>(out) + int64_t(o) * d.out_a.dist;
     }
     s.left = static_cast<uint32_t>(d.n_cols) - s.c0;
     const int S = d.nstages, io = d.io;
@@ -316,7 +345,13 @@ __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, voi
     else
         pair_any<kPairCols, FWD>(d.st[0].R, 0, S == 1, s);
 #pragma unroll 1
-    for (int i = 1; i < S; i++) pair_any<kPairWork, FWD>(d.st[i].R, i, i == S - 1 && direct, s);
+    for (int i = 1; i < S; i++) {
+        const bool last = i == S - 1;
+        if (d.rows || (last && d.runs))
+            pair_any<kPairWorkE, FWD>(d.st[i].R, i, last && direct, s);
+        else
+            pair_any<kPairWorkP, FWD>(d.st[i].R, i, last, s);
+    }
     if (!direct) pair_r2c_post<FWD>(s);
 }
 
@@ -339,110 +374,130 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_tile_kernel(const __grid
     const int words = g.d.buf_words;
     uint32_t t = blockIdx.x;
     if (t < tiles) pair_issue(d, g.d.in, pair_smem + kPairHeadWords, t);
-    cp_async_commit();
     for (int i = 0; t < tiles; t += gridDim.x, i++) {
         const uint32_t tn = t + gridDim.x;
-        // the other buffer was released by the barrier that ended the previous tile
+        cp_async_wait_all();
+        __syncthreads();  // this tile has landed, and the previous one's buffer is free
         if (tn < tiles)
             pair_issue(d, g.d.in, pair_smem + kPairHeadWords + ((i + 1) & 1) * words, tn);
         else
             pdl_launch_dependents();
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
         pair_tile<FWD>(0, kPairHeadWords + (i & 1) * words, g.d.in, g.d.out, t);
-        __syncthreads();
     }
-    cp_async_wait<0>();
 }
 
 // ------------------------------------------------------------------------------------ uneven batches
-// The work list of batch_fft_kernel (fft_tile.cu) on pair tiles: items
-// (segment, tile) are dequeued in order from a global counter, a segment waits
-// (bounded) for every tile of the segment whose output it reads, and the CTA's
-// next item is dequeued and, when its producer has finished, copied in while
-// the current one computes.  Items are ordered so that producers are dequeued
-// before their consumers and every CTA is resident, so the waits end.
-__device__ __forceinline__ bool pair_dep_done(const PairSeg *segs, int *done, int dep)
+// One persistent launch over the work list: CTA b runs items b, b + grid, ...
+// (segment, tile).  A segment waits (bounded) for every tile of the segment
+// whose output it reads.  Items are ordered so that producers come before
+// their consumers and every CTA is resident, so the waits end: the first
+// unfinished item never waits.
+//
+// Everything an item needs is in shared memory before its turn, copied with
+// cp.async under the previous items: its place in the list three items ahead,
+// its descriptor two, its tile one (when its producer has finished; otherwise
+// at its turn).  (Dequeued from a global counter, with the descriptor read at
+// its turn, a chain of four dependent global loads stood between two tiles:
+// barrier and long-scoreboard stalls were 5 of 12 cycles per instruction.)
+// Finished producers are remembered, so a CTA polls each at most once more.
+__device__ __forceinline__ int pair_done_count(const int *done, int dep)
 {
-    if (dep < 0) return true;
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done + dep) : "memory");
-    return v >= static_cast<int>(segs[dep].d.tiles);
+    return v;
 }
-__device__ __forceinline__ bool pair_dep_wait(const PairSeg *segs, int *done, int dep, int *err)
-{
-    for (uint32_t poll = 0; poll < (1u << 24); poll++) {
-        if (pair_dep_done(segs, done, dep)) return true;
-        __nanosleep(128);
-    }
-    atomicExch(err, 2);
-    return false;
-}
+
 template <bool FWD>
 __global__ void __launch_bounds__(kPairThreads, 4)
-    pair_batch_kernel(const PairSeg *__restrict__ segs, const int2 *__restrict__ items, int nitems, int *counter,
-                      int *done, BatchBufs bufs, int *err, int buf_words)
+    pair_batch_kernel(const PairSeg *__restrict__ segs, const int2 *__restrict__ items, int nitems, int *done,
+                      BatchBufs bufs, int *err, int buf_words)
 {
-    // [i & 1]: the item computed in iteration i (the next item's slots are
-    // written while the current item's are still read)
-    __shared__ int2 s_item[2];
-    __shared__ int s_ok, s_pref[2];
+    __shared__ __align__(8) int2 s_item[4];           // item k at [k & 3]
+    __shared__ uint32_t s_known[kPairKnown / 32];     // producers seen finished
+    __shared__ int s_flag;
     const int tid = threadIdx.x;
-    auto dequeue = [&](int slot) {
-        const int w = atomicAdd(counter, 1);
-        int2 it = make_int2(-1, 0);
-        int ready = 0;
-        if (w < nitems) {
-            it = items[w];
-            ready = pair_dep_done(segs, done, segs[it.x].dep);
-        }
-        s_item[slot] = it;
-        s_pref[slot] = ready;
+    const int first = blockIdx.x, stride = gridDim.x;
+    for (int i = tid; i < kPairKnown / 32; i += kPairThreads) s_known[i] = 0u;
+    auto place = [&](int k) {  // list entry of this CTA's item k
+        const int64_t w = first + int64_t(k) * stride;
+        if (tid != 0) return;
+        if (w < nitems)
+            cp_async8(&s_item[k & 3], items + w);
+        else
+            s_item[k & 3] = make_int2(-1, 0);
+    };
+    auto describe = [&](int k) {  // its descriptor (the entry has landed)
+        const int sg = s_item[k & 3].x;
+        if (sg < 0) return;
+        const char *src = reinterpret_cast<const char *>(segs + sg);
+        char *dst = reinterpret_cast<char *>(&pair_slot(k % kPairSlots));
+        for (int i = tid; i < static_cast<int>(sizeof(PairSeg) / 16); i += kPairThreads) cp_async16(dst + 16 * i, src + 16 * i);
     };
     auto source = [&](const PairSeg &g) { return static_cast<const char *>(bufs.p[g.in_buf]) + g.in_off; };
-    // copies slot's segment and, when its producer has finished, starts its tile
-    auto fetch = [&](int slot) {
-        if (s_item[slot].x >= 0) {
-            copy_seg(slot, segs + s_item[slot].x);
-            __syncthreads();
-            const PairSeg &g = pair_slot(slot);
-            if (s_pref[slot])
-                pair_issue(g.d, source(g), pair_smem + kPairHeadWords + slot * buf_words, static_cast<uint32_t>(s_item[slot].y));
+    // is the segment's producer finished?  uniform; with `wait`, polls until it is
+    auto ready = [&](const PairSeg &g, bool wait) -> bool {
+        const int dep = g.dep;
+        if (dep < 0) return true;
+        if (dep < kPairKnown && (s_known[dep >> 5] >> (dep & 31) & 1u)) return true;
+        __syncthreads();  // every thread has read the bit that thread 0 may set
+        if (tid == 0) {
+            bool ok = pair_done_count(done, dep) >= g.dep_tiles;
+            for (uint32_t poll = 0; wait && !ok && poll < (1u << 24); poll++) {
+                __nanosleep(128);
+                ok = pair_done_count(done, dep) >= g.dep_tiles;
+            }
+            if (wait && !ok) atomicExch(err, 2);
+            if (ok && dep < kPairKnown) s_known[dep >> 5] |= 1u << (dep & 31);
+            s_flag = ok ? 1 : 0;
         }
-        cp_async_commit();
+        __syncthreads();
+        return s_flag != 0;
     };
-    if (tid == 0) dequeue(0);
+    auto copy_in = [&](int k) {
+        const PairSeg &g = pair_slot(k % kPairSlots);
+        pair_issue(g.d, source(g), pair_smem + kPairHeadWords + (k & 1) * buf_words, static_cast<uint32_t>(s_item[k & 3].y));
+    };
+    place(0);
+    place(1);
+    place(2);
+    cp_async_wait_all();
     __syncthreads();
-    fetch(0);
-    for (int i = 0; s_item[i & 1].x >= 0; i++) {
-        const int cur = i & 1, nx = cur ^ 1, buf = kPairHeadWords + cur * buf_words;
-        // the previous iteration's item, whose slots and buffer these are, ended with a barrier
-        if (tid == 0) dequeue(nx);
-        __syncthreads();
-        fetch(nx);
-        const PairSeg &g = pair_slot(cur);
-        const int2 it = s_item[cur];
-        bool ok = true;
-        if (!s_pref[cur]) {
-            if (tid == 0) s_ok = pair_dep_wait(segs, done, g.dep, err) ? 1 : 0;
-            __syncthreads();
-            ok = s_ok != 0;
-            if (ok) pair_issue(g.d, source(g), pair_smem + buf, static_cast<uint32_t>(it.y));
-            cp_async_commit();
-            cp_async_wait<0>();
-        } else {
-            cp_async_wait<1>();  // the current item's copies have landed
-        }
-        __syncthreads();
-        if (ok) pair_tile<FWD>(cur, buf, source(g), static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(it.y));
-        __syncthreads();
-        if (ok && tid == 0) {
+    describe(0);
+    describe(1);
+    cp_async_wait_all();
+    __syncthreads();
+    // item 0 is the start of some segment's tiles: prefetched like the others
+    bool staged = s_item[0].x >= 0 && ready(pair_slot(0), false);
+    if (staged) copy_in(0);
+    int publish = -1;  // segment whose tile this CTA finished last
+    for (int k = 0;; k++) {
+        cp_async_wait_all();
+        __syncthreads();  // item k's copies, k+1's descriptor and k+2's entry have landed; item k-1 is done
+        if (publish >= 0 && tid == 0) {
             __threadfence();
-            atomicAdd(done + it.x, 1);
+            atomicAdd(done + publish, 1);
         }
+        if (s_item[k & 3].x < 0) break;
+        const PairSeg &g = pair_slot(k % kPairSlots);
+        const bool more = s_item[(k + 1) & 3].x >= 0;
+        if (more) {
+            place(k + 3);
+            describe(k + 2);
+        }
+        bool ok = true;
+        if (!staged) {
+            ok = ready(g, true);
+            if (ok) copy_in(k);
+            cp_async_wait_all();
+            __syncthreads();
+        }
+        staged = more && ready(pair_slot((k + 1) % kPairSlots), false);
+        if (staged) copy_in(k + 1);
+        if (ok)
+            pair_tile<FWD>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
+                           static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(s_item[k & 3].y));
+        publish = ok && g.consumed ? s_item[k & 3].x : -1;
     }
-    cp_async_wait<0>();
 }
 
 }  // namespace

@@ -185,7 +185,7 @@ struct PairSearch {
     int n;
     bool rows, runs;
     int64_t raw_dist;
-    int max_pairs;
+    int max_pairs, max_buf;
     PairChoice best;
     std::vector<int> cur;
     void leaf()
@@ -193,7 +193,7 @@ struct PairSearch {
         PairDesc q{};
         const int S = static_cast<int>(cur.size());
         for (int P = max_pairs; P >= 1; P = rows ? P - 1 : P / 2) {
-            if (!pair_shape(q, n, cur.data(), S, rows, runs, raw_dist, P)) continue;
+            if (!pair_shape(q, n, cur.data(), S, rows, runs, raw_dist, P, max_buf)) continue;
             const double c = pair_tile_cost(n, cur.data(), S, rows, P, q.buf_words);
             if (c < best.cost) {
                 best.cost = c;
@@ -215,15 +215,15 @@ struct PairSearch {
         }
     }
 };
-PairChoice pair_choice(int n, bool rows, bool runs, int64_t raw_dist, int max_pairs)
+PairChoice pair_choice(int n, bool rows, bool runs, int64_t raw_dist, int max_pairs, int max_buf = kPairBufBytes)
 {
     static std::mutex mu;
-    static std::map<std::tuple<int, bool, bool, int64_t, int>, PairChoice> memo;
+    static std::map<std::tuple<int, bool, bool, int64_t, int, int>, PairChoice> memo;
     std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_tuple(n, rows, runs, raw_dist, max_pairs);
+    const auto key = std::make_tuple(n, rows, runs, raw_dist, max_pairs, max_buf);
     auto it = memo.find(key);
     if (it != memo.end()) return it->second;
-    PairSearch s{n, rows, runs, raw_dist, max_pairs, {}, {}};
+    PairSearch s{n, rows, runs, raw_dist, max_pairs, max_buf, {}, {}};
     // the fewest stages that reach n, and one more
     int fewest = 1;
     for (int64_t m = 16; m < n; m *= 16) fewest++;
@@ -234,13 +234,13 @@ PairChoice pair_choice(int n, bool rows, bool runs, int64_t raw_dist, int max_pa
 
 // Split of F into two passes of pair tiles: the divisor pair of the lowest
 // cost.  False when no pair of lengths has tiles.
-bool pair_split(int64_t F, std::vector<int> &out)
+bool pair_split(int64_t F, int max_buf, std::vector<int> &out)
 {
     double best = 1e29;
     for (int64_t a = 2; a * a <= F; a++) {
         if (F % a || F / a > kMaxPassRadix || F / a > 16 * a) continue;
-        const PairChoice x = pair_choice(static_cast<int>(F / a), false, true, F / a, 32);
-        const PairChoice y = pair_choice(static_cast<int>(a), false, false, a, 32);
+        const PairChoice x = pair_choice(static_cast<int>(F / a), false, true, F / a, 64, max_buf);
+        const PairChoice y = pair_choice(static_cast<int>(a), false, false, a, 64, max_buf);
         if (x.cost + y.cost < best) {
             best = x.cost + y.cost;
             out = {static_cast<int>(F / a), static_cast<int>(a)};
@@ -489,6 +489,8 @@ struct Builder {
         return true;
     }
 
+    int pair_buf() const { return p.pair_buf ? p.pair_buf : kPairBufBytes; }
+
     // columns of a pair tile of length n, 0 if it has none
     static int pair_columns(int n) { return 2 * pair_choice(n, false, false, n, 32).P; }
 
@@ -512,7 +514,7 @@ struct Builder {
         } else if (d.io != IO_C2C || d.in_a.cstride != 1 || d.in_a.cblock != 0 || d.out_a.cblock >= most) {
             return true;
         }
-        const bool runs = !rows && d.out_a.estride == 1;
+        const bool runs = !rows && d.out_a.estride == 1;  // (a single stage stores as it reads)
         // no more pairs than there are, and, in a launch of its own, fewer while there
         // are too few tiles to occupy the SMs (columns keep eight pairs, 128-byte
         // runs; a tile keeps 1024 points)
@@ -528,12 +530,13 @@ struct Builder {
             radices = tuned->radices;
             if (tuned->row_threads > 0 && tuned->row_threads <= 128) P = std::min(P, 4);
         } else {
-            const PairChoice c = pair_choice(d.n, rows, runs, in_dist, P);
+            const PairChoice c = pair_choice(d.n, rows, runs, in_dist, P, pair_buf());
             radices = c.radices;
             P = c.P;
         }
-        while (P >= 1 && !pair_shape(q, d.n, radices.data(), static_cast<int>(radices.size()), rows, runs, in_dist, P)) P /= 2;
-        if (P < 1) return true;
+        while (P >= 1 && !radices.empty() && !pair_shape(q, d.n, radices.data(), static_cast<int>(radices.size()), rows, runs, in_dist, P, pair_buf()))
+            P /= 2;
+        if (P < 1 || radices.empty()) return true;
         const int64_t per_outer = (d.n_cols + 2 * q.P - 1) / (2 * q.P), tiles = per_outer * d.n_outer;
         if (tiles >= most) return true;
         const int per_sm = kernel_blocks_per_sm(pair_kernel_fn(s.forward), kPairThreads, pair_smem(q.buf_words));
@@ -552,6 +555,16 @@ struct Builder {
             q.in_a = Addr{in_dist, in_dist, 1, 0, 0};
             q.out_a = Addr{out_dist, out_dist, 1, 0, 0};
         }
+        // the stages' index arithmetic is 32-bit (a pass of 2^31 points or more keeps the one-transform kernels)
+        const Addr &oa = q.out_a;
+        const int64_t limit = (int64_t(1) << 31) - 1;
+        if (q.in_a.estride > limit || oa.estride > limit || oa.cstride > limit || oa.cjump > limit || oa.cstride + oa.cjump > limit)
+            return true;
+        q.in_es = static_cast<uint32_t>(q.in_a.estride);
+        q.out_es = static_cast<uint32_t>(oa.estride);
+        q.out_cs = static_cast<uint32_t>(oa.cstride);
+        q.out_jump = static_cast<int32_t>(oa.cjump);
+        q.out_delta = static_cast<int32_t>(oa.cblock == 1 ? oa.cstride + oa.cjump : (oa.cblock % 2 ? -1 : oa.cstride));
         q.tw = d.tw;
         if (q.nstages > 1) {
             TablePtr t = get_stage_table(radices.data(), q.nstages, device, &err);
@@ -817,7 +830,8 @@ struct Builder {
         // powers of two: balanced passes on the compile-time engines
         std::vector<int> passes;
         int parts = 2;
-        while (!((F & (F - 1)) != 0 && parts == 2 && pair_split(F, passes)) && !split_passes(F, parts, passes)) {
+        const bool engines = (F & (F - 1)) == 0 && (inner == 1 || inner % 2 == 0) && !p.pair_buf;
+        while (!(!engines && parts == 2 && pair_split(F, pair_buf(), passes)) && !split_passes(F, parts, passes)) {
             if (++parts > 6) {
                 err = "length " + std::to_string(F) + " cannot be split into shared-memory passes";
                 return false;
@@ -1022,6 +1036,8 @@ struct Builder {
             // rows up to 8192 points run as one tile; longer rows as two double-buffered
             // passes, which keep ~16 columns per tile and overlap loads with compute
             // (up to 16384 points where a compile-time engine exists: one row per CTA)
+            if (p.pair_buf && n <= p.max_row_n && pair_choice(static_cast<int>(n), true, false, n, 64, p.pair_buf).P == 0)
+                return add_multipass(n, outer, n, n, src, dst);
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {
                 const float2 *tw = table(n, n);

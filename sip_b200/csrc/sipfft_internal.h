@@ -49,7 +49,7 @@ void static_kernel_fns(std::vector<const void *> &out);
 constexpr int kBatchBlock = 256;
 constexpr int kBatchMaxe = 16;
 constexpr int64_t kBatchMaxRowN = 4096;
-constexpr int64_t kPairMaxRowN = 2048;  // the same for batches on the pair kernel
+constexpr int64_t kPairMaxRowN = 1536;  // the same for batches on the pair kernel (four CTAs per SM)
 const void *batch_kernel_fn(bool forward, bool compact);
 cudaError_t launch_batch(int grid, int block, size_t smem, const BatchSeg *segs, const int2 *items, int nitems,
                          int *counter, int *done, const BatchBufs &bufs, int *err, bool forward, bool compact,
@@ -93,7 +93,7 @@ const void *pair_batch_fn(bool forward);
 void pair_kernel_fns(std::vector<const void *> &out);
 size_t pair_smem(int buf_words);
 cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st);
-cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems, int *counter,
+cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,
                               int *done, const BatchBufs &bufs, int *err, bool forward, cudaStream_t st);
 // t[j * ns + k] = exp(-2 pi i j k / denom), j < rows, k < ns
 cudaError_t fill_outer_twiddles(float2 *t, int64_t rows, int64_t ns, int64_t denom, cudaStream_t st);
@@ -268,6 +268,7 @@ struct Plan {
     int row_smem = 64 * 1024;  // shared memory per CTA the row tiles stay under
     int64_t max_row_n = 1 << 30;  // C2C rows longer than this take the multi-pass path
     int max_maxe = 32;            // largest points per thread a tile may use (tuned choices above are ignored)
+    int pair_buf = 0;  // uneven batch on the pair kernel: every step needs a pair tile with buffers of at most this size
     int max_radix = 16;           // largest radix a tile may use (16 and 12 split below it)
     // inverse STFT plan (asdFftIstftMakePlan): one column C2C step into workspace
     // slot 0 ([channel][frame][n_fft]), then the overlap-add kernel

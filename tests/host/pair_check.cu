@@ -50,7 +50,7 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
     for (int s = 0; s < d.nstages; s++) {
         const PairStage &t = d.st[s];
         const bool last = s == d.nstages - 1;
-        const bool fast_e = rows || (last && runs);
+        const bool fast_e = rows || (last && runs && s > 0);
         const int nb = pair_nb(t.R);
         CHECK(t.tasks == t.nbf * d.P && t.tasks <= kPairThreads * nb);
         std::vector<cd> v(size_t(kPairThreads) * nb * t.R);
@@ -59,15 +59,17 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
             for (int tid = 0; tid < kPairThreads; tid++)
                 for (int b = 0; b < nb; b++) {
                     int i = tid + b * kPairThreads;
-                    const bool on = i < t.tasks;
+                    bool on = i < t.tasks;
                     if (!on) i = 0;
                     int p, j;
-                    if (fast_e) {
+                    if (!fast_e) {
+                        p = tid & (d.P - 1);
+                        j = (tid >> d.lp) + b * (kPairThreads >> d.lp);
+                        CHECK((j < t.nbf) == on);
+                        if (!on) j = 0;
+                    } else {
                         p = t.nbf == 1 ? i : static_cast<int>((uint64_t(uint32_t(i)) * t.nbf_m) >> 32);
                         j = i - p * t.nbf;
-                    } else {
-                        p = i & (d.P - 1);
-                        j = i >> d.lp;
                     }
                     const int q = s == 0 ? j : static_cast<int>((uint64_t(uint32_t(j)) * t.ns_m) >> 32);
                     CHECK(p >= 0 && p < d.P && j >= 0 && j < t.nbf && q == j / t.ns);
@@ -79,7 +81,7 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
                             if (s == 0) {
                                 a[r] = x[p][j + r * t.nbf];
                             } else {
-                                const int at = pair_gather_at(d, t, p, j, q) + r * t.gstep;
+                                const int at = pair_gather_at(d.SP, d.SE, t.gpad, p, j, q) + r * t.gstep;
                                 CHECK(at >= 0 && at < d.buf_words);
                                 a[r] = work[at] * std::polar(1.0, -2 * M_PI * double(r) * k / (double(t.ns) * t.R));
                             }
@@ -91,7 +93,7 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
                     } else if (on) {
                         for (int r = 0; r < t.R; r++) {
                             if (last) got[p][j + r * t.ns] = a[r];  // outputs j + r ns (k = j)
-                            const int at = pair_scatter_at(d, t, p, j, q) + r * t.ns * d.SE;
+                            const int at = pair_scatter_at(d.SP, d.SE, t.spad, t.ns, t.R, p, j, q) + r * t.ns * d.SE;
                             CHECK(at >= 0 && at < d.buf_words);
                             work[at] = a[r];
                         }
