@@ -21,6 +21,7 @@ void pair_kernel_fns(std::vector<const void *> &out)
         out.push_back(pair_kernel_fn(f != 0));
         out.push_back(pair_batch_fn(f != 0));
     }
+    out.push_back(pair_blue_fn());
 }
 
 size_t pair_smem(int buf_words)
@@ -37,6 +38,15 @@ cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t 
     g.d = d;
     void *args[] = {&g};
     return launch_pdl(pair_kernel_fn(forward), dim3(grid), dim3(kPairThreads), smem, st, args);
+}
+
+cudaError_t launch_pair_blue(const PairBlue &q, int grid, cudaStream_t st)
+{
+    const size_t smem = pair_smem(q.g.d.buf_words);
+    if (grid <= 0 || q.g.d.tiles == 0 || smem > static_cast<size_t>(kMaxSmemBytes)) return cudaErrorInvalidConfiguration;
+    PairBlue g = q;
+    void *args[] = {&g};
+    return launch_pdl(pair_blue_fn(), dim3(grid), dim3(kPairThreads), smem, st, args);
 }
 
 cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,

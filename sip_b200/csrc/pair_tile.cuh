@@ -70,6 +70,15 @@ struct alignas(16) PairSeg {
     int dep, dep_tiles, consumed;
 };
 
+// A Bluestein transform in one kernel (pair_blue_kernel): rows of length nb as a
+// circular convolution of length d.n, both FFTs in shared memory.
+struct alignas(16) PairBlue {
+    PairSeg g;  // g.d: rows of d.n points; in / out as for the other kernels
+    const float2 *chirp, *bmul;
+    int64_t in_dist, out_dist;  // float2 (real sides: float) elements between rows
+    int nb, kind;               // TileDesc::blue_n, blue_kind
+};
+
 // Relative cost per point of a tile of P pairs: every thread runs every
 // butterfly slot of a stage (about eight instructions of addressing,
 // shared-memory and twiddle work per point and the butterfly's FP32 operations,

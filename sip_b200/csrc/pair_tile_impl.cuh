@@ -386,6 +386,102 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_tile_kernel(const __grid
     }
 }
 
+// ------------------------------------------------------------------------------------ Bluestein
+// y[k] = chirp[k] IFFT_M(FFT_M(x chirp) bmul)[k] of two rows per thread: one read
+// of x, one write of y, both FFTs in shared memory (as two launches the M-point
+// intermediate went through HBM and the tiles ran on the one-transform kernel:
+// 1021 x 4096 204 us).  The inverse FFT is conj(FFT(conj .)).  Two tile buffers:
+// the first FFT works in one, the product is staged as rows in the other.
+template <int KIND>
+__device__ __forceinline__ float2 blue_in(const void *in, int64_t base, int e, int nb)
+{
+    if constexpr (KIND == 1) {
+        return make_float2(static_cast<const float *>(in)[base + e], 0.f);
+    } else if constexpr (KIND == 2) {
+        const float2 *x = static_cast<const float2 *>(in) + base;
+        if (2 * e > nb) return cconj(x[nb - e]);
+        float2 v = x[e];
+        if (e == 0 || 2 * e == nb) v.y = 0.f;
+        return v;
+    } else {
+        return static_cast<const float2 *>(in)[base + e];
+    }
+}
+
+template <int KIND>
+__device__ __forceinline__ void blue_load(const PairBlue &q, int m, int rows, int64_t row0, float2 *raw)
+{
+    for (int e = threadIdx.x; e < m; e += kPairThreads) {
+        if (e < q.nb) {
+            const float2 c = __ldg(q.chirp + e);
+            for (int l = 0; l < rows; l++) raw[l * m + e] = cmul(blue_in<KIND>(q.g.d.in, (row0 + l) * q.in_dist, e, q.nb), c);
+        } else {
+            for (int l = 0; l < rows; l++) raw[l * m + e] = make_float2(0.f, 0.f);
+        }
+    }
+}
+
+__device__ __forceinline__ void pair_row_stages(const PairTileState &s)
+{
+    const PairDesc &d = pair_slot(s.slot).d;
+    pair_any<kPairRows, true>(d.st[0].R, 0, false, s);
+#pragma unroll 1
+    for (int i = 1; i < d.nstages; i++) pair_any<kPairWorkE, true>(d.st[i].R, i, false, s);
+}
+
+__global__ void __launch_bounds__(kPairThreads, 4) pair_blue_kernel(const __grid_constant__ PairBlue q)
+{
+    copy_seg(0, &q.g);
+    pdl_wait();
+    __syncthreads();
+    const int m = q.g.d.n, P = q.g.d.P, SP = q.g.d.SP, words = q.g.d.buf_words;
+    float4 *A = pair_smem + kPairHeadWords, *B = A + words;
+    for (uint32_t t = blockIdx.x; t < q.g.d.tiles; t += gridDim.x) {
+        const int64_t row0 = int64_t(t) * (2 * P);
+        const int rows = static_cast<int>(min(int64_t(2 * P), q.g.d.n_cols - row0)), pairs = (rows + 1) / 2;
+        float2 *raw = reinterpret_cast<float2 *>(A);
+        if (q.kind == 0)
+            blue_load<0>(q, m, rows, row0, raw);
+        else if (q.kind == 1)
+            blue_load<1>(q, m, rows, row0, raw);
+        else
+            blue_load<2>(q, m, rows, row0, raw);
+        if (t + gridDim.x >= q.g.d.tiles) pdl_launch_dependents();
+        __syncthreads();
+        PairTileState s{0, kPairHeadWords, 0, nullptr, 0u, static_cast<uint32_t>(rows)};
+        pair_row_stages(s);
+        raw = reinterpret_cast<float2 *>(B);
+        for (int e = threadIdx.x; e < m; e += kPairThreads) {
+            const float2 c = __ldg(q.bmul + e);
+            for (int p = 0; p < pairs; p++) {
+                const cpx2 v = cconj(cmul(word_in(A[p * SP + e]), c));
+                raw[2 * p * m + e] = first_of(v);
+                if (2 * p + 1 < rows) raw[(2 * p + 1) * m + e] = second_of(v);
+            }
+        }
+        __syncthreads();
+        s.buf = kPairHeadWords + words;
+        pair_row_stages(s);
+        const int count = q.kind == 1 ? q.nb / 2 + 1 : q.nb;
+        for (int e = threadIdx.x; e < count; e += kPairThreads) {
+            const float2 c = __ldg(q.chirp + e);
+            for (int p = 0; p < pairs; p++) {
+                const cpx2 v = cmul(cconj(word_in(B[p * SP + e])), c);
+                const int64_t y0 = (row0 + 2 * p) * q.out_dist + e;
+                if (q.kind == 2) {
+                    float *y = static_cast<float *>(q.g.d.out);
+                    y[y0] = v.re.x;
+                    if (2 * p + 1 < rows) y[y0 + q.out_dist] = v.re.y;
+                } else {
+                    float2 *y = static_cast<float2 *>(q.g.d.out);
+                    st_stream(y + y0, first_of(v));
+                    if (2 * p + 1 < rows) st_stream(y + y0 + q.out_dist, second_of(v));
+                }
+            }
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------ uneven batches
 // One persistent launch over the work list: CTA b runs items b, b + grid, ...
 // (segment, tile).  A segment waits (bounded) for every tile of the segment

@@ -891,6 +891,28 @@ struct Builder {
             err = "length " + std::to_string(n) + " needs Bluestein with M > " + std::to_string(kMaxBluesteinM);
             return false;
         }
+        // In one kernel where the convolution fits a pair tile, with the cheapest
+        // length among a few times powers of two (planar data and uneven batches
+        // keep tile steps).
+        PairChoice fused;
+        if (p.fft_type != 0x30 && !p.use_tuned && rows < (int64_t(1) << 31)) {
+            const int64_t pow2 = m;
+            double best = 1e30;
+            for (int64_t f : {1, 3, 5, 7, 9, 15}) {
+                int64_t len = f;
+                while (len < 2 * n - 1) len *= 2;
+                if (len > pow2 || len > 2048) continue;
+                int64_t pairs = 16;
+                while (pairs > 1 && (pairs / 2 >= (rows + 1) / 2 || (len * pairs > 1024 && (rows + 1) / 2 < pairs * sm_count(device) * 2)))
+                    pairs /= 2;
+                const PairChoice c = pair_choice(static_cast<int>(len), true, false, len, static_cast<int>(pairs));
+                if (c.P > 0 && c.cost * len < best) {
+                    best = c.cost * len;
+                    fused = c;
+                    m = len;
+                }
+            }
+        }
         const bool multipass = m > kMaxRowN;
         auto chirp = std::make_shared<DeviceTable>();
         auto bmul = std::make_shared<DeviceTable>();
@@ -924,6 +946,7 @@ struct Builder {
         }
         p.tables.push_back(chirp);
         p.tables.push_back(bmul);
+        if (fused.P > 0) return add_bluestein_fused(kind, n, m, rows, in_dist, out_dist, src, dst, chirp->ptr, bmul->ptr, fused);
         if (multipass) return add_bluestein_steps(kind, n, m, rows, in_dist, out_dist, src, dst, chirp->ptr, bmul->ptr);
         Buf ws = other_ws(src, dst);
         need_ws(ws, size_t(rows) * m * sizeof(float2));
@@ -946,6 +969,44 @@ struct Builder {
         s2.forward = false;
         p.steps.push_back(s1);
         p.steps.push_back(s2);
+        return true;
+    }
+
+    bool add_bluestein_fused(int kind, int64_t n, int64_t m, int64_t rows, int64_t in_dist, int64_t out_dist, Buf src,
+                             Buf dst, const float2 *chirp, const float2 *bmul, const PairChoice &c)
+    {
+        Step s;
+        s.kind = StepKind::kBlueFused;
+        s.src = src;
+        s.dst = dst;
+        s.rows = rows;
+        s.m = m;
+        s.src_dist = in_dist;
+        s.dst_dist = out_dist;
+        s.d.blue_n = static_cast<int>(n);
+        s.d.blue_kind = kind;
+        s.d.chirp = chirp;
+        s.d.bmul = bmul;
+        PairDesc &q = s.pd;
+        const int S = static_cast<int>(c.radices.size());
+        if (!pair_shape(q, static_cast<int>(m), c.radices.data(), S, true, false, m, c.P)) {
+            err = "no pair tile for the convolution";
+            return false;
+        }
+        q.io = IO_C2C;
+        q.in_a.dist = m;
+        TablePtr t = get_stage_table(c.radices.data(), S, device, &err);
+        if (!t) return false;
+        p.tables.push_back(t);
+        q.stw = t->ptr;
+        const int per_sm = std::max(1, kernel_blocks_per_sm(pair_blue_fn(), kPairThreads, pair_smem(q.buf_words)));
+        s.pair_grid = per_sm * sm_count(device);
+        std::ostringstream w;
+        w << "Bluestein n=" << n << " via M=" << m << " rows=" << rows << " in one kernel, radices=";
+        for (int i = 0; i < S; i++) w << (i ? "x" : "") << c.radices[i];
+        w << " pairs=" << q.P << " grid=" << s.pair_grid;
+        s.what = w.str();
+        p.steps.push_back(s);
         return true;
     }
 

@@ -388,6 +388,22 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                 e = launch_blue_post(static_cast<const float2 *>(src), dst, s.rows, s.d.blue_n, s.m, s.dst_dist,
                                      s.d.blue_kind, s.d.chirp, st);
                 break;
+            case StepKind::kBlueFused: {
+                PairBlue q{};
+                q.g.d = s.pd;
+                q.g.d.in = src;
+                q.g.d.out = dst;
+                q.g.d.n_cols = s.rows;
+                q.g.d.tiles = static_cast<uint32_t>((s.rows + 2 * s.pd.P - 1) / (2 * s.pd.P));
+                q.chirp = s.d.chirp;
+                q.bmul = s.d.bmul;
+                q.in_dist = s.src_dist;
+                q.out_dist = s.dst_dist;
+                q.nb = s.d.blue_n;
+                q.kind = s.d.blue_kind;
+                e = launch_pair_blue(q, static_cast<int>(std::min<int64_t>(q.g.d.tiles, s.pair_grid)), st);
+                break;
+            }
             case StepKind::kTranspose:
                 e = launch_transpose(static_cast<const float2 *>(src), static_cast<float2 *>(dst), s.t_batch, s.t_rows,
                                      s.t_cols, p.device, st);

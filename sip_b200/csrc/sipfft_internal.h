@@ -90,6 +90,8 @@ cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, size_t smem, int 
 // Runtime-radix tiles of two rows or columns per thread (pair_tile_impl.cuh).
 const void *pair_kernel_fn(bool forward);
 const void *pair_batch_fn(bool forward);
+const void *pair_blue_fn();
+cudaError_t launch_pair_blue(const PairBlue &q, int grid, cudaStream_t st);
 void pair_kernel_fns(std::vector<const void *> &out);
 size_t pair_smem(int buf_words);
 cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st);
@@ -187,7 +189,8 @@ constexpr int kWsSlots = 4;
 // transform whose convolution length M is too long for one CTA (the M-point
 // FFTs between them are multi-pass tile steps).
 enum class StepKind : int {
-    kTile = 0, kR2CPost = 1, kC2RPre = 2, kBluePre = 3, kPointMul = 4, kBluePost = 5, kTranspose = 6
+    kTile = 0, kR2CPost = 1, kC2RPre = 2, kBluePre = 3, kPointMul = 4, kBluePost = 5, kTranspose = 6,
+    kBlueFused = 7  // a whole Bluestein transform in one kernel of pair tiles (pd, pair_grid, d.chirp / bmul)
 };
 
 struct Step {
