@@ -15,6 +15,7 @@ the exec entry point that matches the plan type.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional, Sequence
 
@@ -104,7 +105,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
     vp, i32, i64, u64, sz = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_uint64, ctypes.c_size_t
     P64 = ctypes.POINTER(ctypes.c_int64)
     sig = {
-        "aclCreateTensor": (vp, [P64, u64, ctypes.c_int, P64, i64, ctypes.c_int, P64, u64, vp]),
+        "aclCreateTensor": (vp, [vp, u64, ctypes.c_int, vp, i64, ctypes.c_int, vp, u64, vp]),
         "aclDestroyTensor": (i32, [vp]),
         "aclGetDataType": (i32, [vp, ctypes.POINTER(ctypes.c_int)]),
         "aclGetViewShape": (i32, [vp, ctypes.POINTER(P64), ctypes.POINTER(u64)]),
@@ -235,40 +236,57 @@ def launch_count(handle) -> int:
 
 
 # --- aclTensor -----------------------------------------------------------------------------------
+@functools.lru_cache(maxsize=1024)
+def _dims(shape: tuple) -> tuple:
+    """Number of dimensions, and the extents and contiguous strides as addresses of ctypes
+    arrays (which come last, to keep them); the library copies them."""
+    nd = len(shape)
+    strides = [1] * nd
+    for i in range(nd - 2, -1, -1):
+        strides[i] = strides[i + 1] * shape[i + 1]
+    array = ctypes.c_int64 * max(1, nd)
+    keep = array(*shape), array(*strides)
+    return nd, ctypes.addressof(keep[0]), ctypes.addressof(keep[1]), keep
+
+
+_DTYPES: dict = {}  # torch dtype -> aclDataType, filled at first use
+
+
+def _dtype_code(dtype) -> int:
+    if not _DTYPES:
+        import torch
+
+        _DTYPES.update({torch.complex64: ACL_COMPLEX64, torch.float32: ACL_FLOAT})
+    code = _DTYPES.get(dtype)
+    if code is None:
+        raise TypeError(f"unsupported dtype {dtype}")
+    return code
+
+
 class AclTensor:
     """aclTensor descriptor over a device buffer (shape, dtype, data pointer)."""
 
+    # A small transform's call is bound by the host: its two descriptors took a third of
+    # it when the extents and strides were rebuilt as ctypes arrays every time.
     def __init__(self, shape: Sequence[int], dtype: int, data_ptr: int, owner=None):
-        lib = load_library()
+        lib = _lib if _lib is not None else load_library()
         self.shape = [int(s) for s in shape]
-        nd = len(self.shape)
-        dims = (ctypes.c_int64 * max(1, nd))(*self.shape)
-        strides = [1] * nd
-        for i in range(nd - 2, -1, -1):
-            strides[i] = strides[i + 1] * self.shape[i + 1]
-        st = (ctypes.c_int64 * max(1, nd))(*strides)
-        self.ptr = lib.aclCreateTensor(dims, nd, dtype, st, 0, ACL_FORMAT_ND, dims, nd, ctypes.c_void_p(data_ptr))
+        nd, dims, strides, _ = _dims(tuple(self.shape))
+        self.ptr = lib.aclCreateTensor(dims, nd, dtype, strides, 0, ACL_FORMAT_ND, dims, nd, data_ptr)
         if not self.ptr:
             raise ValueError("aclCreateTensor failed")
         self._owner = owner  # keeps the torch storage alive
 
     @classmethod
     def from_torch(cls, t):
-        import torch
-
-        if t.dtype == torch.complex64:
-            dt = ACL_COMPLEX64
-        elif t.dtype == torch.float32:
-            dt = ACL_FLOAT
-        else:
-            raise TypeError(f"unsupported dtype {t.dtype}")
+        code = _dtype_code(t.dtype)
         if not t.is_contiguous():
             raise ValueError("tensor must be contiguous")
-        return cls(list(t.shape), dt, t.data_ptr(), owner=t)
+        return cls(t.shape, code, t.data_ptr(), owner=t)
 
     def close(self):
         if self.ptr:
-            load_library().aclDestroyTensor(self.ptr)
+            _lib.aclDestroyTensor(self.ptr)
             self.ptr = None
 
     def __del__(self):
@@ -328,14 +346,15 @@ class FftPlan:
         return asdFftSetStream(self.handle, ctypes.c_void_p(stream.cuda_stream))
 
     def __call__(self, inp, out):
-        a, b = AclTensor.from_torch(inp), AclTensor.from_torch(out)
+        a = AclTensor.from_torch(inp)
+        b = AclTensor.from_torch(out)
         try:
             if self.fft_type == ASCEND_FFT_C2C:
-                st = asdFftExecC2C(self.handle, a, b)
+                st = _lib.asdFftExecC2C(self.handle, a.ptr, b.ptr)
             elif self.fft_type == ASCEND_FFT_R2C:
-                st = asdFftExecR2C(self.handle, a, b)
+                st = _lib.asdFftExecR2C(self.handle, a.ptr, b.ptr)
             else:
-                st = asdFftExecC2R(self.handle, a, b)
+                st = _lib.asdFftExecC2R(self.handle, a.ptr, b.ptr)
         finally:
             a.close()
             b.close()
