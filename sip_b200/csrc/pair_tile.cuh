@@ -39,7 +39,7 @@ struct PairDesc {
     int n, io, nstages;
     int P, lp;        // pairs per tile (columns: a power of two and its log2)
     int SE, SP;
-    int pad;          // words inserted every radix[0] elements between stage 0 and 1 (0: none)
+    int descending;   // last tile first (single steps)
     int rows;         // 1: contiguous rows, 0: columns
     int runs;         // last stage walked with the elements fastest (columns stored contiguously)
     int buf_words;    // 16-byte words of one tile buffer
@@ -120,7 +120,6 @@ inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool r
     d.SE = rows ? 1 : (runs ? P | 1 : P);
     const int elems = n + (padded ? n / radix[0] : 0);
     d.SP = rows ? elems | 1 : 1;
-    d.pad = padded ? 1 : 0;
     const int64_t work = rows ? int64_t(P - 1) * d.SP + elems : int64_t(elems - 1) * d.SE + P;
     const int64_t raw = rows ? (2 * P * raw_dist + 3) / 2 : int64_t(n) * P;
     const int64_t words = ((work > raw ? work : raw) + 7) / 8 * 8;

@@ -372,17 +372,18 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_tile_kernel(const __grid
     const PairDesc &d = pair_slot(0).d;
     const uint32_t tiles = g.d.tiles;
     const int words = g.d.buf_words;
+    auto at = [&](uint32_t t) { return g.d.descending ? tiles - 1 - t : t; };
     uint32_t t = blockIdx.x;
-    if (t < tiles) pair_issue(d, g.d.in, pair_smem + kPairHeadWords, t);
+    if (t < tiles) pair_issue(d, g.d.in, pair_smem + kPairHeadWords, at(t));
     for (int i = 0; t < tiles; t += gridDim.x, i++) {
         const uint32_t tn = t + gridDim.x;
         cp_async_wait_all();
         __syncthreads();  // this tile has landed, and the previous one's buffer is free
         if (tn < tiles)
-            pair_issue(d, g.d.in, pair_smem + kPairHeadWords + ((i + 1) & 1) * words, tn);
+            pair_issue(d, g.d.in, pair_smem + kPairHeadWords + ((i + 1) & 1) * words, at(tn));
         else
             pdl_launch_dependents();
-        pair_tile<FWD>(0, kPairHeadWords + (i & 1) * words, g.d.in, g.d.out, t);
+        pair_tile<FWD>(0, kPairHeadWords + (i & 1) * words, g.d.in, g.d.out, at(t));
     }
 }
 

@@ -449,6 +449,10 @@ struct Builder {
         }
         if (column && io == IO_C2C && !add_column_variant(s)) return false;
         if (!add_pair_variant(s, tuned ? &tc : nullptr)) return false;
+        // against the step before it; the columns of a 2D C2R plan, whose rows end the
+        // plan in ascending order, start at the end
+        if (s.cp_fn || (s.pair && !s.row_fn))
+            s.descending = p.steps.empty() ? p.fft_type == 0x11 && p.sizes.size() == 2 : !p.steps.back().descending;
         // passes of a multi-pass transform keep the FP32 kernels: their tiles would run on the
         // single-tile tensor-core kernel, several times slower than the double-buffered FP32 passes
         if (in_multipass || p.fft_type == 0x30 || !(io == IO_C2C || io == IO_R2C_PACKED || io == IO_C2R_PACKED))

@@ -326,6 +326,7 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                     PairDesc d = s.pd;
                     d.in = src;
                     d.out = dst;
+                    d.descending = s.descending ? 1 : 0;
                     e = launch_pair(d, s.forward, s.pair_grid, st);
                 } else if (s.has_row && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && src != dst) {
                     TileDesc d = s.rd;
@@ -340,12 +341,13 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                     TileDesc d = s.cd;
                     d.in = src;
                     d.out = dst;
-                    e = launch_col_pipe(s.cp_fn, d, s.cp_smem, s.cp_grid, device_error_word(p.device), st);
+                    e = launch_col_pipe(s.cp_fn, d, s.cp_smem, s.cp_grid, s.descending, device_error_word(p.device), st);
                 } else if (s.pair && (!s.pd.rows || src != dst)) {
                     // a source that the static engines' bulk copies cannot read
                     PairDesc d = s.pd;
                     d.in = src;
                     d.out = dst;
+                    d.descending = s.descending ? 1 : 0;
                     e = launch_pair(d, s.forward, s.pair_grid, st);
                 } else if (s.db) {
                     TileDesc d = s.d;

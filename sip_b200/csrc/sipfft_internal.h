@@ -86,7 +86,8 @@ bool col_pipe_has_engine(int n);  // a TMA column engine exists for this length
 void col_pipe_kernel_fns(std::vector<const void *> &out);
 // the step's input addressing and sizes fit the tensor map of the column kernel
 bool col_pipe_layout_ok(const TileDesc &d);
-cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, size_t smem, int grid, int *err, cudaStream_t st);
+cudaError_t launch_col_pipe(const void *fn, const TileDesc &d, size_t smem, int grid, bool descending, int *err,
+                            cudaStream_t st);
 // Runtime-radix tiles of two rows or columns per thread (pair_tile_impl.cuh).
 const void *pair_kernel_fn(bool forward);
 const void *pair_batch_fn(bool forward);
@@ -212,6 +213,9 @@ struct Step {
     int cp_grid = 1;
     size_t cp_smem = 0;
     TileDesc cd{};
+    // column and pair kernels: last tile first (each step walks against the one
+    // before it, whose last outputs are still in L2)
+    bool descending = false;
     // runtime-radix pair tiles (no alignment requirement)
     bool pair = false;
     PairDesc pd{};
