@@ -194,7 +194,7 @@ ColPipeEntry col_entry()
 const std::vector<ColPipeEntry> &col_registry()
 {
     static const std::vector<ColPipeEntry> r = {
-        col_entry<Seq<16, 4>, 4, 16>(),     col_entry<Seq<16, 8>, 8, 16>(),    col_entry<Seq<16, 16>, 16, 8>(),
+        col_entry<Seq<16, 2>, 2, 32>(),     col_entry<Seq<16, 4>, 4, 16>(),     col_entry<Seq<16, 8>, 8, 16>(),    col_entry<Seq<16, 16>, 16, 8>(),
         col_entry<Seq<16, 16, 2>, 32, 4>(), col_entry<Seq<16, 16, 4>, 64, 2>(), col_entry<Seq<16, 16, 8>, 128, 2, true>(),
     };
     return r;

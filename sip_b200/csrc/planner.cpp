@@ -506,6 +506,10 @@ struct Builder {
         const bool rows = !d.xfast;
         const int64_t most = int64_t(1) << 31;
         if (d.n < 2 || d.n_cols >= most || d.n_outer >= most) return true;
+        // Columns with a compile-time engine keep it: the TMA tiles, and for strides those
+        // cannot read (odd ones, as the half spectra of R2C plans have) the element-copy
+        // tiles (r2c 512^2 x 16 28 us, 32 on pair tiles; 128^2 x 256 29, 30)
+        if ((s.cp_fn || s.db_fn) && !p.use_tuned) return true;
         int64_t in_dist = d.in_a.dist, out_dist = d.out_a.dist, max_pairs = 64;
         if (rows) {
             if (!(d.io == IO_C2C || d.io == IO_R2C_PACKED || d.io == IO_C2R_PACKED) || d.n_outer != 1 ||
@@ -1103,6 +1107,15 @@ struct Builder {
             // (up to 16384 points where a compile-time engine exists: one row per CTA)
             if (p.pair_buf && n <= p.max_row_n && pair_choice(static_cast<int>(n), true, false, n, 64, p.pair_buf).P == 0)
                 return add_multipass(n, outer, n, n, src, dst);
+            // Above 4096 points a row and its double buffer leave one CTA per SM: even lengths
+            // without a compile-time engine take two passes of pair tiles (7680 x 1024
+            // 126 -> 64 us, 5000 x 2048 123 -> 108, 4320 x 2048 95 -> 81; odd ones, whose
+            // columns copy 8 bytes at a time, stay: 6561 x 1024 73 us, 97 in two passes).
+            if (n > 4096 && n <= kMaxSingleTileC2C && n % 2 == 0 && !p.use_tuned && p.precision == 0 &&
+                !find_static_kernel(static_cast<int>(n), IO_C2C)) {
+                std::vector<int> two;
+                if (pair_split(n, kPairBufBytes, two)) return add_multipass(n, outer, n, n, src, dst);
+            }
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {
                 const float2 *tw = table(n, n);
@@ -1127,7 +1140,7 @@ struct Builder {
             if ((form == 1 || form == 2) && tc_rows_config(static_cast<int>(n), tcc))
                 return add_transposed_axis(n, outer, inner, src, dst);
             if (form == 0 && !p.vertical && n > 256 && n <= kMaxStridedTile && inner > 1 &&
-                !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
+                !(n <= 1024 && find_static_kernel(static_cast<int>(n), IO_C2C)) && !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
                 return add_multipass(n, outer, n * inner, n * inner, src, dst, inner);
         }
         TileCfg c;
