@@ -256,32 +256,54 @@ __device__ __forceinline__ void pair_any(int R, int stage, bool to_global, const
 #undef SIPFFT_PAIR
 }
 
+// The real kinds' passes over the pairs of bins k and m-k of every row hold
+// kRealUnroll pairs in flight per thread.
+constexpr int kRealUnroll = 4;
+
 // R2C post-twiddle of the packed transforms in the work tile: bins k and m-k
 // of every row (r2c_pair on two rows at once).
 template <bool FWD>
 __device__ __noinline__ void pair_r2c_post(const PairTileState s)
 {
     const PairDesc &d = pair_slot(s.slot).d;
-    const int m = d.n, half = m / 2 + 1;
+    const int m = d.n, half = m / 2 + 1, SP = d.SP;
     const int64_t dist = d.out_a.dist;
-    const uint32_t total = static_cast<uint32_t>(half * d.P);
-    for (uint32_t i = threadIdx.x; i < total; i += kPairThreads) {
-        const int p = static_cast<int>(d.dv_post.div(i)), k = static_cast<int>(i) - p * half;
-        if (static_cast<uint32_t>(2 * p) >= s.left) break;
-        const float4 *w = pair_smem + s.buf + p * d.SP;
-        const cpx2 zk = word_in(w[k]), zm = word_in(w[k == 0 ? 0 : m - k]);
-        // X[k] = S/2 + w U/2, X[m-k] = conj(S/2 - w U/2), S = Z[k] + conj Z[m-k], U = -i (Z[k] - conj Z[m-k])
-        const cpx2 S = cscale(cadd(zk, cconj(zm)), 0.5f);
-        const cpx2 D = cscale(csub(zk, cconj(zm)), 0.5f);
-        const cpx2 wu = cmul(cneg(mul_i(D)), dir<FWD>(__ldg(d.tw + k)));
-        const cpx2 a = cadd(S, wu), b = cconj(csub(S, wu));
-        float2 *y = s.out + (s.c0 + 2 * p) * dist;
-        const bool second = static_cast<uint32_t>(2 * p + 1) < s.left;
-        st_stream(y + k, first_of(a));
-        if (second) st_stream(y + dist + k, second_of(a));
-        if (2 * k != m) {
-            st_stream(y + m - k, first_of(b));
-            if (second) st_stream(y + dist + m - k, second_of(b));
+    const FastDiv by_half = d.dv_post;
+    const float2 *tw = d.tw;
+    // (the pairs of rows that exist)
+    const uint32_t total = static_cast<uint32_t>(half) * min(static_cast<uint32_t>(d.P), (s.left + 1) / 2);
+    for (uint32_t i0 = threadIdx.x; i0 < total; i0 += kRealUnroll * kPairThreads) {
+        cpx2 zk[kRealUnroll], zm[kRealUnroll];
+        float2 w[kRealUnroll];
+#pragma unroll
+        for (int u = 0; u < kRealUnroll; u++) {
+            const uint32_t i = min(i0 + u * kPairThreads, total - 1);
+            const int p = static_cast<int>(by_half.div(i)), k = static_cast<int>(i) - p * half;
+            const float4 *z = pair_smem + s.buf + p * SP;
+            zk[u] = word_in(z[k]);
+            zm[u] = word_in(z[k == 0 ? 0 : m - k]);
+            w[u] = __ldg(tw + k);
+        }
+#pragma unroll
+        for (int u = 0; u < kRealUnroll; u++) {
+            const uint32_t i = i0 + u * kPairThreads;
+            if (i < total) {
+                const int p = static_cast<int>(by_half.div(i)), k = static_cast<int>(i) - p * half;
+                // X[k] = S/2 + w U/2, X[m-k] = conj(S/2 - w U/2), S = Z[k] + conj Z[m-k], U = -i (Z[k] - conj Z[m-k])
+                const cpx2 S = cscale(cadd(zk[u], cconj(zm[u])), 0.5f);
+                const cpx2 D = cscale(csub(zk[u], cconj(zm[u])), 0.5f);
+                const cpx2 wu = cmul(cneg(mul_i(D)), dir<FWD>(w[u]));
+                const cpx2 a = cadd(S, wu), b = cconj(csub(S, wu));
+                float2 *y = s.out + (s.c0 + 2 * p) * dist + k;
+                const bool second = static_cast<uint32_t>(2 * p + 1) < s.left, both_bins = 2 * k != m;
+                st_stream(y, first_of(a));
+                if (both_bins) st_stream(y + (m - 2 * k), first_of(b));
+                if (second) {
+                    y += dist;
+                    st_stream(y, second_of(a));
+                    if (both_bins) st_stream(y + (m - 2 * k), second_of(b));
+                }
+            }
         }
     }
 }
@@ -293,22 +315,41 @@ __device__ __noinline__ void pair_c2r_pre(const PairTileState s)
 {
     const PairDesc &d = pair_slot(s.slot).d;
     const int m = d.n, half = m / 2 + 1, dist = static_cast<int>(d.in_a.dist);
-    const uint32_t total = static_cast<uint32_t>(half * d.P);
-    for (uint32_t i = threadIdx.x; i < total; i += kPairThreads) {
-        const int p = static_cast<int>(d.dv_post.div(i)), k = static_cast<int>(i) - p * half;
-        if (static_cast<uint32_t>(2 * p) >= s.left) break;
-        float2 *x0 = reinterpret_cast<float2 *>(pair_smem + s.buf) + s.mis + (2 * p) * dist;
-        float2 *x1 = static_cast<uint32_t>(2 * p + 1) < s.left ? x0 + dist : x0;
-        cpx2 xk = pair_of(x0[k], x1[k]), xm = pair_of(x0[m - k], x1[m - k]);
-        if (k == 0) xk.im = xm.im = make_float2(0.f, 0.f);
-        const cpx2 ev = cadd(xk, cconj(xm));
-        const cpx2 od = cmul(csub(xk, cconj(xm)), dir<FWD>(__ldg(d.tw + k)));
-        const cpx2 zk = cadd_i(ev, od), zm = cconj(csub_i(ev, od));
-        x0[k] = first_of(zk);
-        x1[k] = second_of(zk);
-        if (k != 0 && 2 * k != m) {
-            x0[m - k] = first_of(zm);
-            x1[m - k] = second_of(zm);
+    const FastDiv by_half = d.dv_post;
+    const float2 *tw = d.tw;
+    const uint32_t total = static_cast<uint32_t>(half) * min(static_cast<uint32_t>(d.P), (s.left + 1) / 2);
+    float2 *raw = reinterpret_cast<float2 *>(pair_smem + s.buf) + s.mis;
+    for (uint32_t i0 = threadIdx.x; i0 < total; i0 += kRealUnroll * kPairThreads) {
+        cpx2 xk[kRealUnroll], xm[kRealUnroll];
+        float2 w[kRealUnroll];
+        // a pair of bins is read and written by one thread only; the clamped rounds
+        // beyond `total` read the last pair and write nothing
+#pragma unroll
+        for (int u = 0; u < kRealUnroll; u++) {
+            const uint32_t i = min(i0 + u * kPairThreads, total - 1);
+            const int p = static_cast<int>(by_half.div(i)), k = static_cast<int>(i) - p * half;
+            const float2 *x0 = raw + (2 * p) * dist, *x1 = static_cast<uint32_t>(2 * p + 1) < s.left ? x0 + dist : x0;
+            xk[u] = pair_of(x0[k], x1[k]);
+            xm[u] = pair_of(x0[m - k], x1[m - k]);
+            w[u] = __ldg(tw + k);
+        }
+#pragma unroll
+        for (int u = 0; u < kRealUnroll; u++) {
+            const uint32_t i = i0 + u * kPairThreads;
+            if (i < total) {
+                const int p = static_cast<int>(by_half.div(i)), k = static_cast<int>(i) - p * half;
+                float2 *x0 = raw + (2 * p) * dist, *x1 = static_cast<uint32_t>(2 * p + 1) < s.left ? x0 + dist : x0;
+                if (k == 0) xk[u].im = xm[u].im = make_float2(0.f, 0.f);
+                const cpx2 ev = cadd(xk[u], cconj(xm[u]));
+                const cpx2 od = cmul(csub(xk[u], cconj(xm[u])), dir<FWD>(w[u]));
+                const cpx2 zk = cadd_i(ev, od), zm = cconj(csub_i(ev, od));
+                x0[k] = first_of(zk);
+                x1[k] = second_of(zk);
+                if (k != 0 && 2 * k != m) {
+                    x0[m - k] = first_of(zm);
+                    x1[m - k] = second_of(zm);
+                }
+            }
         }
     }
 }
