@@ -355,7 +355,8 @@ __device__ __noinline__ void pair_c2r_pre(const PairTileState s)
 }
 
 // Stages of one staged tile (a barrier after its copies is the caller's).
-template <bool FWD>
+// REAL: the descriptor may be a packed real kind (not in the uneven batch).
+template <bool FWD, bool REAL>
 __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, void *out, uint32_t t)
 {
     const PairDesc &d = pair_slot(slot).d;
@@ -374,10 +375,12 @@ __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, voi
     }
     s.left = static_cast<uint32_t>(d.n_cols) - s.c0;
     const int S = d.nstages, io = d.io;
-    const bool direct = io != IO_R2C_PACKED;  // R2C: the post-twiddle writes the outputs
-    if (io == IO_C2R_PACKED) {
-        pair_c2r_pre<FWD>(s);
-        __syncthreads();
+    const bool direct = !REAL || io != IO_R2C_PACKED;  // R2C: the post-twiddle writes the outputs
+    if constexpr (REAL) {
+        if (io == IO_C2R_PACKED) {
+            pair_c2r_pre<FWD>(s);
+            __syncthreads();
+        }
     }
     if (d.rows)
         pair_any<kPairRows, FWD>(d.st[0].R, 0, S == 1 && direct, s);
@@ -393,7 +396,9 @@ __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, voi
         else
             pair_any<kPairWorkP, FWD>(d.st[i].R, i, last, s);
     }
-    if (!direct) pair_r2c_post<FWD>(s);
+    if constexpr (REAL) {
+        if (!direct) pair_r2c_post<FWD>(s);
+    }
 }
 
 __device__ __forceinline__ void copy_seg(int slot, const PairSeg *src)
@@ -424,7 +429,7 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_tile_kernel(const __grid
             pair_issue(d, g.d.in, pair_smem + kPairHeadWords + ((i + 1) & 1) * words, at(tn));
         else
             pdl_launch_dependents();
-        pair_tile<FWD>(0, kPairHeadWords + (i & 1) * words, g.d.in, g.d.out, at(t));
+        pair_tile<FWD, true>(0, kPairHeadWords + (i & 1) * words, g.d.in, g.d.out, at(t));
     }
 }
 
@@ -672,7 +677,7 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         staged = more && ready(pair_slot((k + 1) % kPairSlots), false);
         if (staged) copy_in(k + 1);
         if (ok)
-            pair_tile<FWD>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
+            pair_tile<FWD, false>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
                            static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(s_item[k & 3].y));
         publish = ok && g.consumed ? s_item[k & 3].x : -1;
     }

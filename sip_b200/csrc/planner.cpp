@@ -192,7 +192,12 @@ struct PairSearch {
     {
         PairDesc q{};
         const int S = static_cast<int>(cur.size());
-        for (int P = max_pairs; P >= 1; P = rows ? P - 1 : P / 2) {
+        int P = max_pairs;  // the threads' butterflies bound it
+        for (int R : cur) {
+            const int fit = kPairThreads * pair_nb(R) / (n / R);
+            while (P > fit && P > 0) P = rows ? fit : P / 2;
+        }
+        for (; P >= 1; P = rows ? P - 1 : P / 2) {
             if (!pair_shape(q, n, cur.data(), S, rows, runs, raw_dist, P, max_buf)) continue;
             const double c = pair_tile_cost(n, cur.data(), S, rows, P, q.buf_words);
             if (c < best.cost) {
@@ -200,7 +205,8 @@ struct PairSearch {
                 best.radices = cur;
                 best.P = P;
             }
-            if (!rows) break;  // fewer columns never pay
+            // fewer pairs never pay, but for the buffer size of four CTAs per SM
+            if (!rows || q.buf_words * 16 <= kPairBufBytes4) break;
         }
     }
     void walk(int m, int most, int stages_left)
@@ -411,6 +417,7 @@ struct Builder {
         d.out_a = oa;
         d.tw = tw;
         d.tw_mul = tw_mul;
+        if (p.pair_buf) return add_pair_variant(s, tuned ? &tc : nullptr);  // no other kernel runs it
         if (d.nstages > 1) {
             // contiguous per-stage twiddles: coalesced reads in every stage
             TablePtr st = get_stage_table(d.radix, d.nstages, device, &err);
@@ -862,8 +869,8 @@ struct Builder {
             Buf nxt = last ? dst : other_ws(cur, dst);
             const int64_t nxt_dist = last ? out_dist : F * inner;
             if (!last) need_ws(nxt, size_t(outer) * F * inner * sizeof(float2));
-            const float2 *tw = table(rp, rp);
-            if (!tw) return false;
+            const float2 *tw = p.pair_buf ? nullptr : table(rp, rp);  // (pair tiles of C2C steps do not read it)
+            if (!tw && !p.pair_buf) return false;
             Addr ia{cur_dist, 1, (F / rp) * inner, 0, 0};
             Addr oa{nxt_dist, 1, ns * inner, ns * inner, ns * inner * (rp - 1)};
             std::ostringstream w;
@@ -1118,8 +1125,8 @@ struct Builder {
             }
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {
-                const float2 *tw = table(n, n);
-                if (!tw) return false;
+                const float2 *tw = p.pair_buf ? nullptr : table(n, n);
+                if (!tw && !p.pair_buf) return false;
                 Addr a{0, n, 1, 0, 0};
                 return add_tile(IO_C2C, static_cast<int>(n), 1, tw, false, 1, outer, a, a, src, dst, w.str());
             }
@@ -1131,8 +1138,11 @@ struct Builder {
         }
         // Tensor-core forms of lengths with the row pipeline: through transposes.
         // FP32 axes without a TMA column engine whose pair tile would keep at most
-        // four columns (32-byte row runs, lengths above about 512): as two passes of
-        // pair tiles, which keep 16 and more.  Vertical 1D plans keep their column
+        // four columns (32-byte row runs, lengths above about 400): as two passes of
+        // pair tiles, which keep 16 and more (us, transposes or column tiles of one
+        // transform per thread -> two passes: 1080 x 1920 x 8 378 -> 180, 1000^2 x 16
+        // 322 -> 175, 4096^2 x 1 203 -> 163, 2048^2 r2c x 4 120 -> 107); 512 and 1024
+        // points with odd strides keep the element-copy tiles of their engines.  Vertical 1D plans keep their column
         // tiles (complex32 data converts in the first and last tile steps).
         if (!in_multipass && p.fft_type != 0x30) {
             TcConfig tcc;
@@ -1140,7 +1150,8 @@ struct Builder {
             if ((form == 1 || form == 2) && tc_rows_config(static_cast<int>(n), tcc))
                 return add_transposed_axis(n, outer, inner, src, dst);
             if (form == 0 && !p.vertical && n > 256 && n <= kMaxStridedTile && inner > 1 &&
-                !(n <= 1024 && find_static_kernel(static_cast<int>(n), IO_C2C)) && !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
+                !(n <= 1024 && find_static_kernel(static_cast<int>(n), IO_C2C)) &&
+                !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
                 return add_multipass(n, outer, n * inner, n * inner, src, dst, inner);
         }
         TileCfg c;
