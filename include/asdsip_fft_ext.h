@@ -52,9 +52,14 @@ ASDSIP_API int32_t asdFftBatchPlanCreate(void **plan, const int64_t *sizes, cons
                                          int32_t direction, const char *tune_cache);
 ASDSIP_API int32_t asdFftBatchGetWorkspaceSize(void *plan, size_t *bytes);
 /* in != out; workspace of GetWorkspaceSize bytes; stream = cudaStream_t; use_graph != 0 captures once and
- * replays while (in, out, workspace, stream) stay the same. */
+ * replays while (in, out, workspace, stream) stay the same.  A tile waits for the tiles it reads for a bounded
+ * number of polls (environment variable ASDSIP_FFT_BATCH_POLLS at plan creation, of at least 128 ns each; default
+ * 2^24).  When a wait gives up, the call's results are incomplete: the next Exec of the plan, or Synchronize,
+ * returns ACL_ERROR_INTERNAL_ERROR once (that Exec launches nothing). */
 ASDSIP_API int32_t asdFftBatchExec(void *plan, const void *input, void *output, void *workspace, void *stream,
                                    int32_t use_graph);
+/* Waits for the stream (cudaStream_t) and reports a call whose results are incomplete. */
+ASDSIP_API int32_t asdFftBatchSynchronize(void *plan, void *stream);
 ASDSIP_API int32_t asdFftBatchPlanDestroy(void *plan);
 ASDSIP_API int64_t asdFftBatchDescribe(void *plan, char *buf, int64_t len);
 

@@ -6,8 +6,9 @@
 // An uneven batch is a list of groups (length n_i, count b_i) of 1D C2C
 // transforms stored back to back.  Every group is planned with the ordinary
 // planner; its launches become segments of one work list (segment, tile)
-// executed by a single persistent kernel (batch_fft_kernel in fft_tile.cu),
-// whose CTAs dequeue tiles from a global counter.  A segment that reads
+// executed by a single persistent kernel (pair_batch_kernel in
+// pair_tile_impl.cuh; batch_fft_kernel in fft_tile.cu for sets with a Bluestein
+// length or a length of one), whose CTAs take tiles from a global counter.  A segment that reads
 // another segment's output (the next pass of a long transform, the second
 // half of a Bluestein transform) waits for that segment's completion count.
 // The counter reset and the launch are captured once into a CUDA graph and
@@ -232,7 +233,9 @@ struct BatchPlan {
     PairSeg *d_pair_segs = nullptr;
     int buf_words = 0;  // tile buffer of the pair kernel
     int2 *d_items = nullptr;
-    int *d_counters = nullptr;  // [0] = item counter, [1 + s] = tiles done of segment s
+    int *d_counters = nullptr;  // kBatchTicket, kBatchGaveUp, kBatchDone + segment
+    int *status = nullptr;      // mapped host word, set by a kernel whose wait gave up
+    uint32_t polls = kBatchPolls;
     size_t ws_bytes = 0;
     int grid = 1, block = kBatchBlock;
     bool compact = false;  // every segment's radices are <= kCompactMaxRadix (three CTAs per SM)
@@ -255,7 +258,17 @@ struct BatchPlan {
         cudaFree(d_pair_segs);
         cudaFree(d_items);
         cudaFree(d_counters);
+        cudaFreeHost(status);
         cudaGetLastError();
+    }
+    // Reads and clears the status word: true when a call since the last look left its
+    // results incomplete.
+    bool gave_up()
+    {
+        volatile int *w = status;
+        const bool bad = *w != 0;
+        if (bad) *w = 0;
+        return bad;
     }
 };
 
@@ -381,13 +394,19 @@ std::string build_batch_with(BatchPlan &bp)
             return "twiddle table: device allocation failed";
         }
     }
+    if (cudaHostAlloc(&bp.status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return "twiddle table: host allocation failed";
+    }
+    *bp.status = 0;
+    if (const char *s = std::getenv("ASDSIP_FFT_BATCH_POLLS")) bp.polls = static_cast<uint32_t>(std::atoll(s));
     size_t bytes = bp.segs.size() * sizeof(BatchSeg);
     if (cudaMalloc(&bp.d_segs, bytes) != cudaSuccess ||
         cudaMemcpy(bp.d_segs, bp.segs.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&bp.d_items, bp.items.size() * sizeof(int2)) != cudaSuccess ||
         cudaMemcpy(bp.d_items, bp.items.data(), bp.items.size() * sizeof(int2), cudaMemcpyHostToDevice) !=
             cudaSuccess ||
-        cudaMalloc(&bp.d_counters, (1 + bp.segs.size()) * sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&bp.d_counters, (kBatchDone + bp.segs.size()) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         return "twiddle table: device allocation failed";
     }
@@ -419,15 +438,17 @@ std::string build_batch(BatchPlan &bp)
 
 cudaError_t enqueue(BatchPlan &bp, const void *in, void *out, void *ws, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(bp.d_counters, 0, (1 + bp.segs.size()) * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(bp.d_counters, 0, (kBatchDone + bp.segs.size()) * sizeof(int), st);
     if (e != cudaSuccess) return e;
-    BatchBufs bufs{{const_cast<void *>(in), out, ws, nullptr}};
+    BatchBufs bufs{{const_cast<void *>(in), out, ws, nullptr}, nullptr};
+    e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&bufs.status), bp.status, 0);
+    if (e != cudaSuccess) return e;
     if (bp.pairs)
         return launch_pair_batch(bp.grid, bp.buf_words, bp.d_pair_segs, bp.d_items, static_cast<int>(bp.items.size()),
-                                 bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, st);
+                                 bp.d_counters, bufs, device_error_word(bp.device), bp.polls, bp.forward, st);
     return launch_batch(bp.grid, bp.block, bp.smem, bp.d_segs, bp.d_items, static_cast<int>(bp.items.size()),
-                        bp.d_counters, bp.d_counters + 1, bufs, device_error_word(bp.device), bp.forward, bp.compact,
-                        st);
+                        bp.d_counters + kBatchTicket, bp.d_counters + kBatchDone, bufs, device_error_word(bp.device),
+                        bp.forward, bp.compact, st);
 }
 
 std::mutex g_batch_mu;
@@ -720,6 +741,10 @@ int32_t asdFftBatchExec(void *plan, const void *input, void *output, void *works
     if ((reinterpret_cast<uintptr_t>(input) & 7) || (reinterpret_cast<uintptr_t>(output) & 7))
         return AsdSip::ACL_ERROR_INVALID_PARAM;
     std::lock_guard<std::mutex> lock(bp->mu);
+    if (bp->gave_up()) {
+        sipfft::set_last_error("asdFftBatchExec: a wait of an earlier call gave up; that call's results are incomplete");
+        return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
     if (!use_graph) {
@@ -762,6 +787,24 @@ int32_t asdFftBatchExec(void *plan, const void *input, void *output, void *works
     if (e != cudaSuccess) {
         sipfft::set_last_error(std::string("asdFftBatchExec: ") + cudaGetErrorString(e));
         cudaGetLastError();
+        return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+    }
+    return AsdSip::ACL_SUCCESS;
+}
+
+int32_t asdFftBatchSynchronize(void *plan, void *stream)
+{
+    BatchPlan *bp = sipfft::find_batch(plan);
+    if (!bp) return AsdSip::ACL_ERROR_INVALID_PARAM;
+    cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) {
+        sipfft::set_last_error(std::string("asdFftBatchSynchronize: ") + cudaGetErrorString(e));
+        cudaGetLastError();
+        return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+    }
+    std::lock_guard<std::mutex> lock(bp->mu);
+    if (bp->gave_up()) {
+        sipfft::set_last_error("asdFftBatchSynchronize: a wait gave up; the results are incomplete");
         return AsdSip::ACL_ERROR_INTERNAL_ERROR;
     }
     return AsdSip::ACL_SUCCESS;

@@ -274,13 +274,15 @@ __device__ __forceinline__ bool batch_dep_done(const BatchSeg *segs, int *done, 
     return v >= segs[sg.dep].ntiles;
 }
 
-__device__ __forceinline__ bool batch_dep_wait(const BatchSeg *segs, int *done, const BatchSeg &sg, int *err)
+__device__ __forceinline__ bool batch_dep_wait(const BatchSeg *segs, int *done, const BatchSeg &sg, int *err,
+                                               int *status)
 {
-    for (uint32_t poll = 0; poll < (1u << 24); poll++) {
+    for (uint32_t poll = 0; poll < kBatchPolls; poll++) {
         if (batch_dep_done(segs, done, sg)) return true;
         __nanosleep(128);
     }
     atomicExch(err, 2);
+    *static_cast<volatile int *>(status) = 2;
     return false;
 }
 
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(kBatchBlock, COMPACT ? 3 : 2)
         char *out = static_cast<char *>(bufs.p[sg.out_buf]) + sg.out_off;
         bool ok = true;
         if (!pref) {
-            if (tid == 0) s_ok = batch_dep_wait(segs, done, sg, err) ? 1 : 0;
+            if (tid == 0) s_ok = batch_dep_wait(segs, done, sg, err, bufs.status) ? 1 : 0;
             __syncthreads();
             ok = s_ok != 0;
         }

@@ -177,6 +177,12 @@ struct BatchSeg {
 
 struct BatchBufs {
     void *p[4];
+    int *status;  // mapped host word of the plan, set when a wait gave up
 };
+
+// Device words of an uneven batch, cleared before each launch: the next entry of
+// the work list, whether a wait gave up, and the finished tiles of each segment.
+constexpr int kBatchTicket = 0, kBatchGaveUp = 1, kBatchDone = 2;
+constexpr uint32_t kBatchPolls = 1u << 24;  // polls of at least 128 ns before a wait gives up
 
 }  // namespace sipfft

@@ -50,10 +50,10 @@ cudaError_t launch_pair_blue(const PairBlue &q, int grid, cudaStream_t st)
 }
 
 cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,
-                              int *done, const BatchBufs &bufs, int *err, bool forward, cudaStream_t st)
+                              int *words, const BatchBufs &bufs, int *err, uint32_t polls, bool forward, cudaStream_t st)
 {
     BatchBufs b = bufs;
-    void *args[] = {&segs, &items, &nitems, &done, &b, &err, &buf_words};
+    void *args[] = {&segs, &items, &nitems, &words, &b, &err, &buf_words, &polls};
     return cudaLaunchKernel(pair_batch_fn(forward), dim3(grid), dim3(kPairThreads), args, pair_smem(buf_words), st);
 }
 

@@ -570,18 +570,22 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_blue_kernel(const __grid
 }
 
 // ------------------------------------------------------------------------------------ uneven batches
-// One persistent launch over the work list: CTA b runs items b, b + grid, ...
-// (segment, tile).  A segment waits (bounded) for every tile of the segment
-// whose output it reads.  Items are ordered so that producers come before
-// their consumers and every CTA is resident, so the waits end: the first
-// unfinished item never waits.
+// One persistent launch over the work list of (segment, tile) items.  A segment
+// waits (bounded) for every tile of the segment whose output it reads; items are
+// ordered so that producers come before their consumers.  A CTA takes its items
+// from a counter and works them in the order of their tickets, so the waits end
+// however many CTAs run at once: the first unfinished item of the list is the
+// current item of a running CTA (or nobody's yet, and then no CTA waits), and
+// every item that it could wait for comes before it.  (Items dealt by CTA number
+// would need the whole grid resident, which other work on the GPU can prevent.)
 //
-// Everything an item needs is in shared memory before its turn, copied with
-// cp.async under the previous items: its place in the list three items ahead,
-// its descriptor two, its tile one (when its producer has finished; otherwise
-// at its turn).  (Dequeued from a global counter, with the descriptor read at
-// its turn, a chain of four dependent global loads stood between two tiles:
-// barrier and long-scoreboard stalls were 5 of 12 cycles per instruction.)
+// Everything an item needs is in shared memory before its turn: its ticket is
+// drawn four items ahead, its place in the list is copied (cp.async) three items
+// ahead, its descriptor two, its tile one (when its producer has finished;
+// otherwise at its turn).  (With all of that at its turn, a chain of four
+// dependent global loads stood between two tiles: barrier and long-scoreboard
+// stalls were 5 of 12 cycles per instruction.)  The first tickets are drawn one
+// at a time, a load apart, so that short lists spread over the CTAs.
 // Finished producers are remembered, so a CTA polls each at most once more.
 __device__ __forceinline__ int pair_done_count(const int *done, int dep)
 {
@@ -590,24 +594,44 @@ __device__ __forceinline__ int pair_done_count(const int *done, int dep)
     return v;
 }
 
+// Polls of thread 0 until `tiles` tiles of segment dep are finished; false when it
+// gives up, or another CTA has, and the words that say so are set.  (A function of
+// its own: its registers would spill those of the stages.)
+__device__ __noinline__ bool pair_wait(int *words, int dep, int tiles, uint32_t polls, int *err, int *status)
+{
+    for (uint32_t i = 0; i < polls; i++) {
+        __nanosleep(128);
+        if (pair_done_count(words + kBatchDone, dep) >= tiles) return true;
+        if (i % 64 == 63 && *static_cast<volatile int *>(words + kBatchGaveUp) != 0) break;
+    }
+    atomicExch(words + kBatchGaveUp, 1);
+    atomicExch(err, 2);
+    *static_cast<volatile int *>(status) = 2;
+    return false;
+}
+
 template <bool FWD>
 __global__ void __launch_bounds__(kPairThreads, 4)
-    pair_batch_kernel(const PairSeg *__restrict__ segs, const int2 *__restrict__ items, int nitems, int *done,
-                      BatchBufs bufs, int *err, int buf_words)
+    pair_batch_kernel(const PairSeg *__restrict__ segs, const int2 *__restrict__ items, int nitems, int *words,
+                      BatchBufs bufs, int *err, int buf_words, uint32_t polls)
 {
     __shared__ __align__(8) int2 s_item[4];           // item k at [k & 3]
     __shared__ uint32_t s_known[kPairKnown / 32];     // producers seen finished
     __shared__ int s_flag;
     const int tid = threadIdx.x;
-    const int first = blockIdx.x, stride = gridDim.x;
+    uint32_t ticket = 0;  // thread 0: the list entry that this CTA takes next
+    auto draw = [&] {
+        if (tid == 0) ticket = atomicAdd(reinterpret_cast<unsigned *>(words + kBatchTicket), 1u);
+    };
+    draw();
     for (int i = tid; i < kPairKnown / 32; i += kPairThreads) s_known[i] = 0u;
-    auto place = [&](int k) {  // list entry of this CTA's item k
-        const int64_t w = first + int64_t(k) * stride;
+    auto place = [&](int k) {  // list entry of this CTA's item k, and the ticket of item k + 1
         if (tid != 0) return;
-        if (w < nitems)
-            cp_async8(&s_item[k & 3], items + w);
+        if (ticket < static_cast<uint32_t>(nitems))
+            cp_async8(&s_item[k & 3], items + ticket);
         else
             s_item[k & 3] = make_int2(-1, 0);
+        draw();
     };
     auto describe = [&](int k) {  // its descriptor (the entry has landed)
         const int sg = s_item[k & 3].x;
@@ -624,12 +648,8 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         if (dep < kPairKnown && (s_known[dep >> 5] >> (dep & 31) & 1u)) return true;
         __syncthreads();  // every thread has read the bit that thread 0 may set
         if (tid == 0) {
-            bool ok = pair_done_count(done, dep) >= g.dep_tiles;
-            for (uint32_t poll = 0; wait && !ok && poll < (1u << 24); poll++) {
-                __nanosleep(128);
-                ok = pair_done_count(done, dep) >= g.dep_tiles;
-            }
-            if (wait && !ok) atomicExch(err, 2);
+            bool ok = pair_done_count(words + kBatchDone, dep) >= g.dep_tiles;
+            if (wait && !ok) ok = pair_wait(words, dep, g.dep_tiles, polls, err, bufs.status);
             if (ok && dep < kPairKnown) s_known[dep >> 5] |= 1u << (dep & 31);
             s_flag = ok ? 1 : 0;
         }
@@ -641,24 +661,24 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         pair_issue(g.d, source(g), pair_smem + kPairHeadWords + (k & 1) * buf_words, static_cast<uint32_t>(s_item[k & 3].y));
     };
     place(0);
-    place(1);
-    place(2);
     cp_async_wait_all();
     __syncthreads();
     describe(0);
-    describe(1);
+    place(1);
     cp_async_wait_all();
     __syncthreads();
     // item 0 is the start of some segment's tiles: prefetched like the others
     bool staged = s_item[0].x >= 0 && ready(pair_slot(0), false);
     if (staged) copy_in(0);
+    describe(1);
+    place(2);
     int publish = -1;  // segment whose tile this CTA finished last
     for (int k = 0;; k++) {
         cp_async_wait_all();
         __syncthreads();  // item k's copies, k+1's descriptor and k+2's entry have landed; item k-1 is done
         if (publish >= 0 && tid == 0) {
             __threadfence();
-            atomicAdd(done + publish, 1);
+            atomicAdd(words + kBatchDone + publish, 1);
         }
         if (s_item[k & 3].x < 0) break;
         const PairSeg &g = pair_slot(k % kPairSlots);
@@ -667,20 +687,19 @@ __global__ void __launch_bounds__(kPairThreads, 4)
             place(k + 3);
             describe(k + 2);
         }
-        bool ok = true;
         if (!staged) {
-            ok = ready(g, true);
-            if (ok) copy_in(k);
+            if (!ready(g, true)) break;  // the whole CTA: the results are incomplete, and reported as such
+            copy_in(k);
             cp_async_wait_all();
             __syncthreads();
         }
         staged = more && ready(pair_slot((k + 1) % kPairSlots), false);
         if (staged) copy_in(k + 1);
-        if (ok)
-            pair_tile<FWD, false>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
-                           static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(s_item[k & 3].y));
-        publish = ok && g.consumed ? s_item[k & 3].x : -1;
+        pair_tile<FWD, false>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
+                              static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(s_item[k & 3].y));
+        publish = g.consumed ? s_item[k & 3].x : -1;
     }
+    cp_async_wait_all();
 }
 
 }  // namespace

@@ -97,7 +97,8 @@ void pair_kernel_fns(std::vector<const void *> &out);
 size_t pair_smem(int buf_words);
 cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st);
 cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,
-                              int *done, const BatchBufs &bufs, int *err, bool forward, cudaStream_t st);
+                              int *words, const BatchBufs &bufs, int *err, uint32_t polls, bool forward,
+                              cudaStream_t st);
 // t[j * ns + k] = exp(-2 pi i j k / denom), j < rows, k < ns
 cudaError_t fill_outer_twiddles(float2 *t, int64_t rows, int64_t ns, int64_t denom, cudaStream_t st);
 cudaError_t fill_stage_twiddles(float2 *t, const int *radix, int nstages, cudaStream_t st);

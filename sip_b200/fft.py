@@ -65,7 +65,7 @@ EXPORTED_SYMBOLS = (
     "asdFftSynchronize", "asdFftGetType",
     "asdFftExecRaw", "asdFftDescribePlan", "asdFftPlanLaunchCount",
     "asdFftBatchPlanCreate", "asdFftBatchGetWorkspaceSize", "asdFftBatchExec", "asdFftBatchPlanDestroy",
-    "asdFftBatchDescribe", "asdFftAutotune", "asdFftTuneCacheLoad",
+    "asdFftBatchSynchronize", "asdFftBatchDescribe", "asdFftAutotune", "asdFftTuneCacheLoad",
     "asdFftServerCreate", "asdFftServerWarm", "asdFftServerSubmit", "asdFftServerDrain", "asdFftServerBatches",
     "asdFftServerDestroy", "asdFftServeRun", "asdFftServerHold", "asdFftGetErrorMessage",
     "asdFftExecC2CNoAlloc", "asdFftSetPrecision", "asdFftServerSetPrecision",
@@ -135,6 +135,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
         "asdFftBatchPlanCreate": (i32, [ctypes.POINTER(vp), P64, P64, i32, i32, ctypes.c_char_p]),
         "asdFftBatchGetWorkspaceSize": (i32, [vp, ctypes.POINTER(sz)]),
         "asdFftBatchExec": (i32, [vp, vp, vp, vp, vp, i32]),
+        "asdFftBatchSynchronize": (i32, [vp, vp]),
         "asdFftBatchPlanDestroy": (i32, [vp]),
         "asdFftBatchDescribe": (i64, [vp, ctypes.c_char_p, i64]),
         "asdFftAutotune": (i32, [P64, P64, i32, i32, ctypes.c_char_p]),
@@ -420,6 +421,15 @@ class BatchPlan:
         if st != ACL_SUCCESS:
             raise FftError("asdFftBatchExec", st)
         return out
+
+    def synchronize(self, stream=None):
+        """Waits for the stream; raises when a call left its results incomplete."""
+        import torch
+
+        s = stream if stream is not None else torch.cuda.current_stream()
+        st = load_library().asdFftBatchSynchronize(self.handle, ctypes.c_void_p(s.cuda_stream))
+        if st != ACL_SUCCESS:
+            raise FftError("asdFftBatchSynchronize", st)
 
     def describe(self) -> str:
         lib = load_library()
