@@ -99,7 +99,9 @@ AspbStatus finish_plan(sipfft::Plan &p, std::string (*builder)(sipfft::Plan &), 
     p.steps.clear();
     p.tables.clear();
     p.c32_steps.clear();
+    p.c32_base.clear();
     p.c32_state = 0;
+    p.pair_route = false;
     for (size_t &b : p.ws_buf_bytes) b = 0;
     if (builder != sipfft::build_plan_istft) p.istft = false;
     p.ws_bytes = 0;

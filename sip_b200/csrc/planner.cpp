@@ -287,6 +287,9 @@ struct Builder {
     std::string err;
     bool in_multipass = false;  // planning the passes of a multi-pass transform
 
+    // the first and last step run on the generic tile kernel (Plan::tile_ends)
+    bool tile_ends() const { return p.tile_ends || p.fft_type == 0x30; }
+
     const float2 *table(int64_t count, int64_t denom, int64_t mult = 1)
     {
         TablePtr t = get_table(count, denom, mult, device, &err);
@@ -842,15 +845,23 @@ struct Builder {
     bool add_multipass(int64_t F, int64_t outer, int64_t in_dist, int64_t out_dist, Buf src, Buf dst,
                        int64_t inner = 1)
     {
-        // powers of two: balanced passes on the compile-time engines
-        std::vector<int> passes;
+        // powers of two: balanced passes on the compile-time engines; so are the passes of
+        // data that the generic tile kernel reads and writes (separated planes, 1000000 x 4
+        // 152 us, 166 in the split of the pair tiles; complex32 9000 x 466 102, 112)
+        std::vector<int> passes, pairs;
         int parts = 2;
         const bool engines = (F & (F - 1)) == 0 && (inner == 1 || inner % 2 == 0) && !p.pair_buf;
-        while (!(!engines && parts == 2 && pair_split(F, pair_buf(), passes)) && !split_passes(F, parts, passes)) {
-            if (++parts > 6) {
-                err = "length " + std::to_string(F) + " cannot be split into shared-memory passes";
-                return false;
-            }
+        while (!split_passes(F, parts, passes)) {
+            if (++parts > 6) break;
+        }
+        if (!engines && !tile_ends() && pair_split(F, pair_buf(), pairs)) {
+            if (pairs != passes) p.pair_route = true;
+            passes = pairs;
+            parts = 2;
+        }
+        if (parts > 6) {
+            err = "length " + std::to_string(F) + " cannot be split into shared-memory passes";
+            return false;
         }
         const float2 *lo = nullptr, *hi = nullptr;
         int log2l = 0;
@@ -1118,10 +1129,14 @@ struct Builder {
             // without a compile-time engine take two passes of pair tiles (7680 x 1024
             // 126 -> 64 us, 5000 x 2048 123 -> 108, 4320 x 2048 95 -> 81; odd ones, whose
             // columns copy 8 bytes at a time, stay: 6561 x 1024 73 us, 97 in two passes).
-            if (n > 4096 && n <= kMaxSingleTileC2C && n % 2 == 0 && !p.use_tuned && p.precision == 0 &&
+            // Complex32 and separated data stay as well (5000 x 838 52 us, 114; 54, 142).
+            if (n > 4096 && n <= kMaxSingleTileC2C && n % 2 == 0 && !p.use_tuned && p.precision == 0 && !tile_ends() &&
                 !find_static_kernel(static_cast<int>(n), IO_C2C)) {
                 std::vector<int> two;
-                if (pair_split(n, kPairBufBytes, two)) return add_multipass(n, outer, n, n, src, dst);
+                if (pair_split(n, kPairBufBytes, two)) {
+                    p.pair_route = true;
+                    return add_multipass(n, outer, n, n, src, dst);
+                }
             }
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {
@@ -1377,7 +1392,24 @@ std::string build_plan_1d(Plan &p)
         default:
             b.err = "unsupported transform type";
     }
-    return finish(p, b, ok);
+    std::string e = finish(p, b, ok);
+    if (!e.empty() || !p.pair_route || p.fft_type != 0x10 || p.use_tuned || p.precision != 0) return e;
+    // a plan of interleaved data may be run on complex32 data: its steps where the route differs
+    Plan half;
+    half.fft_type = p.fft_type;
+    half.direction = p.direction;
+    half.sizes = p.sizes;
+    half.strides = p.strides;
+    half.batch = p.batch;
+    half.vertical = p.vertical;
+    half.device = p.device;
+    half.tile_ends = true;
+    e = build_plan_1d(half);
+    if (!e.empty()) return e;
+    p.c32_base = half.steps;
+    p.tables.insert(p.tables.end(), half.tables.begin(), half.tables.end());
+    for (int i = 0; i < kWsSlots; i++) p.ws_buf_bytes[i] = std::max(p.ws_buf_bytes[i], half.ws_buf_bytes[i]);
+    return finish(p, b, true);
 }
 
 std::string build_plan_2d(Plan &p)
@@ -1487,6 +1519,10 @@ std::string describe_plan(const Plan &p)
                   << " grid=" << s.row_grid << " smem=" << row_kernel_smem(s.rd);
         }
         o << "\n";
+    }
+    if (!p.c32_base.empty()) {
+        o << "complex32 data: steps=" << p.c32_base.size() << "\n";
+        for (const Step &s : p.c32_base) o << "  " << s.what << "\n";
     }
     return o.str();
 }

@@ -214,7 +214,7 @@ std::string complex32_steps(const Plan &p, std::vector<Step> &out)
 {
     if (p.fft_type != 0x10 || p.sizes.size() != 1) return "complex32 data is supported for 1D C2C plans";
     if (p.precision != 0) return "complex32 data runs with FP32 stages only (precision mode 0)";
-    out = p.steps;
+    out = p.c32_base.empty() ? p.steps : p.c32_base;
     if (out.empty()) return "empty plan";
     for (size_t i = 0; i < out.size(); i++) {
         Step &s = out[i];

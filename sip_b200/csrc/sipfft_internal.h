@@ -278,6 +278,10 @@ struct Plan {
     int max_maxe = 32;            // largest points per thread a tile may use (tuned choices above are ignored)
     int pair_buf = 0;  // uneven batch on the pair kernel: every step needs a pair tile with buffers of at most this size
     int max_radix = 16;           // largest radix a tile may use (16 and 12 split below it)
+    // The first and last step run on the generic tile kernel, the only one that reads and
+    // writes complex32 and separated data: routes that pay on the pair kernels are not taken.
+    bool tile_ends = false;
+    bool pair_route = false;  // (set by the planner) such a route was taken
     // inverse STFT plan (asdFftIstftMakePlan): one column C2C step into workspace
     // slot 0 ([channel][frame][n_fft]), then the overlap-add kernel
     bool istft = false;
@@ -288,6 +292,7 @@ struct Plan {
     int precision = 0;
     // complex32 (FP16 pairs) variant of a 1D C2C plan's steps, built at the
     // first complex32 exec (c32_state: 0 not built, 1 built, -1 unsupported)
+    std::vector<Step> c32_base;  // the steps that it converts, where not `steps` (pair_route)
     std::vector<Step> c32_steps;
     int c32_state = 0;
     bool forward() const;

@@ -1,0 +1,73 @@
+"""GPU: calls that stay off the kernels of two transforms per thread where those lose, each
+against the FP64 oracle on the route that its plan names."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from sip_b200 import fft
+
+pytestmark = pytest.mark.gpu
+
+C2C, R2C, C2R, SEP = fft.ASCEND_FFT_C2C, fft.ASCEND_FFT_R2C, fft.ASCEND_FFT_C2R, fft.ASCEND_FFT_C2C_SEP
+FWD, INV = fft.ASCEND_FFT_FORWARD, fft.ASCEND_FFT_INVERSE
+VERT, HORI = fft.ASCEND_FFT_VERTICAL, fft.ASCEND_FFT_HORIZONTAL
+
+
+@pytest.mark.parametrize("n", [4098 + 18, 5000, 7680, 8190])
+@pytest.mark.parametrize("direction", [FWD, INV])
+def test_separated_long_even_rows_in_one_launch(cuda, n, direction):
+    import torch
+
+    rng = np.random.default_rng(n)
+    re, im = rng.uniform(-1, 1, (2, 5, n)).astype(np.float32)
+    h = fft.asdFftCreate()
+    try:
+        assert fft.asdFftMakePlan1D(h, n, SEP, direction, 5) == fft.ACL_SUCCESS
+        assert fft.launch_count(h) == 1, fft.describe_plan(h)
+        assert fft.asdFftGetWorkspaceSize(h) == (fft.ACL_SUCCESS, 0)
+        fft.asdFftSetStream(h, torch.cuda.current_stream().cuda_stream or 1)
+        x = [torch.from_numpy(v).cuda() for v in (re, im)]
+        y = [torch.empty_like(v) for v in x]
+        t = [fft.AclTensor.from_torch(v) for v in x + y]
+        assert fft.load_library().asdFftExecC2CSeparated(h, *[v.ptr for v in t]) == fft.ACL_SUCCESS
+        torch.cuda.synchronize()
+        got = y[0].cpu().numpy() + 1j * y[1].cpu().numpy()
+        assert oracle.rel_l2(got, oracle.c2c(re + 1j * im, direction == FWD)) <= oracle.tolerance(n)
+    finally:
+        fft.asdFftDestroy(h)
+
+
+@pytest.mark.parametrize("n,batch,vertical,steps", [(4116, 5, False, 1), (5000, 4, False, 1), (8190, 3, False, 1),
+                                                    (9000, 3, False, 2), (1000000, 1, False, 2), (9000, 7, True, 2)])
+@pytest.mark.parametrize("direction", [FWD, INV])
+def test_complex32_route(cuda, n, batch, vertical, steps, direction):
+    """complex32 data takes the tile kernel's own route (FP16 in and out, FP32 between): the
+    result is the FP64 one to the rounding of the outputs, 2^-11 relative each; 1e-3 as for
+    the other lengths."""
+    import torch
+
+    rng = np.random.default_rng(n + batch)
+    shape = (n, batch) if vertical else (batch, n)
+    xh = rng.uniform(-1, 1, shape + (2,)).astype(np.float16)
+    xd = torch.from_numpy(xh).cuda()
+    yd = torch.full_like(xd, float("nan"))
+    plan = fft.FftPlan([n], C2C, direction, batch, VERT if vertical else HORI)
+    assert f"complex32 data: steps={steps}" in plan.describe(), plan.describe()
+    a = fft.AclTensor(shape, fft.ACL_COMPLEX32, xd.data_ptr())
+    b = fft.AclTensor(shape, fft.ACL_COMPLEX32, yd.data_ptr())
+    assert fft.asdFftExecC2C(plan.handle, a, b) == fft.ACL_SUCCESS
+    torch.cuda.synchronize()
+    y = yd.cpu().numpy().astype(np.float64)
+    x = xh.astype(np.float64)
+    x, got = x[..., 0] + 1j * x[..., 1], y[..., 0] + 1j * y[..., 1]
+    ref = oracle.c2c(x.T, direction == FWD).T if vertical else oracle.c2c(x, direction == FWD)
+    assert oracle.rel_l2(got, ref) <= 1e-3
+    # interleaved FP32 data of the same plan
+    xc = torch.from_numpy(x.astype(np.complex64)).cuda()
+    yc = torch.empty_like(xc)
+    plan(xc, yc)
+    torch.cuda.synchronize()
+    assert oracle.rel_l2(yc.cpu().numpy(), ref) <= oracle.tolerance(n)
+    for t in (a, b):
+        t.close()
+    plan.close()
