@@ -527,6 +527,10 @@ struct Builder {
                 return true;
             in_dist = d.in_a.cstride;
             out_dist = d.out_a.cstride;
+            // Rows of a few points: a tile's fixed work is spread over too little, and the
+            // one-transform tile kernel is faster (4 M points, us, pair tiles -> tile kernel: c2c
+            // 2 points 51 -> 31, 5 28 -> 23, 12 31 -> 26, 13 26 -> 25, 14 equal; r2c 8 20 -> 15).
+            if (d.n < 14 && !p.use_tuned) return true;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
         } else if (d.io != IO_C2C || d.in_a.cstride != 1 || d.in_a.cblock != 0 || d.out_a.cblock >= most) {

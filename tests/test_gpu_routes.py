@@ -71,3 +71,38 @@ def test_complex32_route(cuda, n, batch, vertical, steps, direction):
     for t in (a, b):
         t.close()
     plan.close()
+
+
+def _check(sizes, typ, direction, batch, seed, vertical=False):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    fwd, nd = direction == FWD, len(sizes)
+    shape = [sizes[0], batch] if vertical else [batch] + list(sizes)
+    if typ == R2C:
+        x = rng.standard_normal(shape).astype(np.float32)
+        ref = oracle.r2c(x, fwd, nd)
+    elif typ == C2R:
+        shape[-1] = sizes[-1] // 2 + 1
+        x = (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)).astype(np.complex64)
+        ref = oracle.c2r(x, sizes[-1], fwd, nd)
+    else:
+        x = (rng.uniform(-1, 1, shape) + 1j * rng.uniform(-1, 1, shape)).astype(np.complex64)
+        ref = oracle.c2c(x.T, fwd).T if vertical else oracle.c2c(x, fwd, nd)
+    plan = fft.FftPlan(sizes, typ, direction, batch, VERT if vertical else HORI)
+    y = torch.empty(ref.shape, dtype=torch.complex64 if np.iscomplexobj(ref) else torch.float32, device="cuda")
+    plan(torch.from_numpy(np.ascontiguousarray(x)).cuda(), y)
+    torch.cuda.synchronize()
+    assert oracle.rel_l2(y.cpu().numpy(), ref) <= oracle.tolerance(int(np.prod(sizes))), plan.describe()
+    text = plan.describe()
+    plan.close()
+    return text
+
+
+@pytest.mark.parametrize("n", list(range(2, 17)))
+@pytest.mark.parametrize("direction", [FWD, INV])
+def test_short_rows(cuda, n, direction):
+    """Rows of fewer than 14 points (packed points of real rows) on the tile kernel."""
+    for typ, k in ((C2C, n), (R2C, 2 * n), (C2R, 2 * n)):
+        text = _check([k], typ, direction, 1031, seed=n)
+        assert ("[pair tiles]" in text) == (n >= 14 and "static" not in text), text
