@@ -533,6 +533,11 @@ struct Builder {
             if (d.n < 14 && !p.use_tuned) return true;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
+        } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32)) {
+            // Few short columns (one tile per outer index, of a few hundred points at most): the
+            // one-transform tiles put more CTAs on an SM (4 M points, us, pair tiles / those: 8 x 8
+            // 1.95, 16 x 12 1.44, 30 x 9 1.43, 20 x 5 2.0; 36 x 9 1.0, 16 x 24 0.91, 8 x 33 0.90).
+            return true;
         } else if (d.io != IO_C2C || d.in_a.cstride != 1 || d.in_a.cblock != 0 || d.out_a.cblock >= most) {
             return true;
         }

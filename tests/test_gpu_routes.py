@@ -106,3 +106,18 @@ def test_short_rows(cuda, n, direction):
     for typ, k in ((C2C, n), (R2C, 2 * n), (C2R, 2 * n)):
         text = _check([k], typ, direction, 1031, seed=n)
         assert ("[pair tiles]" in text) == (n >= 14 and "static" not in text), text
+
+
+@pytest.mark.parametrize("xy", [(3, 7), (8, 8), (8, 33), (9, 16), (9, 17), (16, 12), (16, 24), (30, 9), (32, 16), (33, 9),
+                                (36, 2)])
+@pytest.mark.parametrize("direction", [FWD, INV])
+def test_short_narrow_columns(cuda, xy, direction):
+    """Columns of up to 32 points, at most 16 of them (32 below 9 points), on the tile kernel."""
+    x, y = xy
+    text = _check([x, y], C2C, direction, 21, seed=x)
+    columns = [l for l in text.splitlines() if "[1->1]" in l]
+    assert len(columns) == 1
+    few = x <= 32 and y <= (16 if x >= 9 else 32)
+    assert ("[pair tiles]" in columns[0]) == (not few), text
+    _check([x, 2 * y], R2C, direction, 21, seed=x)
+    _check([x, 2 * y], C2R, direction, 21, seed=x)
