@@ -928,9 +928,11 @@ struct Builder {
         }
         // In one kernel where the convolution fits a pair tile, with the cheapest
         // length among a few times powers of two (planar data and uneven batches
-        // keep tile steps).
+        // keep tile steps).  Convolutions of up to 64 points keep them too: the row by
+        // row element-wise passes cost more than the saved intermediate (4 M points, us,
+        // one kernel / two launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317).
         PairChoice fused;
-        if (p.fft_type != 0x30 && !p.use_tuned && rows < (int64_t(1) << 31)) {
+        if (p.fft_type != 0x30 && !p.use_tuned && 2 * n - 1 > 64 && rows < (int64_t(1) << 31)) {
             const int64_t pow2 = m;
             double best = 1e30;
             for (int64_t f : {1, 3, 5, 7, 9, 15}) {

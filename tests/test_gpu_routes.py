@@ -121,3 +121,12 @@ def test_short_narrow_columns(cuda, xy, direction):
     assert ("[pair tiles]" in columns[0]) == (not few), text
     _check([x, 2 * y], R2C, direction, 21, seed=x)
     _check([x, 2 * y], C2R, direction, 21, seed=x)
+
+
+@pytest.mark.parametrize("n", [17, 23, 31, 34, 37])
+@pytest.mark.parametrize("direction", [FWD, INV])
+def test_short_bluestein(cuda, n, direction):
+    """Convolutions of up to 64 points in two launches, longer ones in one kernel."""
+    for typ in (C2C, R2C, C2R):
+        text = _check([n], typ, direction, 333, seed=n)
+        assert ("in one kernel" in text) == (2 * n - 1 > 64), text
