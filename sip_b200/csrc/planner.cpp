@@ -239,10 +239,10 @@ PairChoice pair_choice(int n, bool rows, bool runs, int64_t raw_dist, int max_pa
 }
 
 // Split of F into two passes of pair tiles: the divisor pair of the lowest
-// cost.  False when no pair of lengths has tiles.
-bool pair_split(int64_t F, int max_buf, std::vector<int> &out)
+// cost (`best`).  False when no pair of lengths has tiles.
+bool pair_split(int64_t F, int max_buf, std::vector<int> &out, double &best)
 {
-    double best = 1e29;
+    best = 1e29;
     for (int64_t a = 2; a * a <= F; a++) {
         if (F % a || F / a > kMaxPassRadix || F / a > 16 * a) continue;
         const PairChoice x = pair_choice(static_cast<int>(F / a), false, true, F / a, 64, max_buf);
@@ -605,6 +605,31 @@ struct Builder {
         return true;
     }
 
+    // Rows of 4097..8192 points without a compile-time engine, `outer` of them: two passes of pair
+    // tiles, or one tile.  Odd lengths stay in one, since their columns copy 8 bytes at a time
+    // (6561 x 1024 73 us, 97 in two passes).  Measured over every even length (13-smooth), us, one
+    // tile -> two passes, at 2^22 and 2^25 points unless stated:
+    // * above about 6800 points a row and its double buffer leave one CTA per SM, and five stages
+    //   take the tile as long: two passes (7680 67 -> 32 and 430 -> 236, 6000 56 -> 41 and 350 -> 292);
+    // * while the data, its intermediate and the result take half of L2, the two passes' smaller
+    //   tiles occupy the SMs better: every length (4374 at 2^18 points 16 -> 11, 5000 20 -> 11);
+    // * else by the cost of the split, while all three fit L2 (cost 205: 4374 43 -> 56 at 262,
+    //   5082 43 -> 52 at 209, 6552 55 -> 46 at 185), and not for lengths near 4096 whose passes
+    //   have an odd distance (4410 45 -> 49);
+    // * beyond L2 the second pass's traffic shows: only multiples of 16, whose passes keep
+    //   16-byte copies and whole sectors (4410 297 -> 338, 6084 274 -> 331; 4368 322 -> 282).
+    bool long_row_in_two(int64_t n, int64_t outer) const
+    {
+        std::vector<int> one, two;
+        double cost;
+        if (n % 2 || !factor_radices(n, one) || !pair_split(n, kPairBufBytes, two, cost)) return false;
+        constexpr int64_t kL2 = int64_t(126) << 20;
+        const int64_t bytes = 3 * int64_t(sizeof(float2)) * n * outer;
+        if (n >= 6800 || one.size() >= 5 || bytes <= kL2 / 2) return true;
+        if (bytes <= kL2) return cost <= 205 && (two[1] % 2 == 0 || n % 8 == 0 || n >= 4500);
+        return cost <= 190 && n % 16 == 0;
+    }
+
     // Inter-pass twiddle tables of a kernel of two columns per thread whose
     // first radix is r0: t1 up to 8 MB (beyond it the rows of t1 come from the
     // two-level table), t2 always.
@@ -863,7 +888,8 @@ struct Builder {
         while (!split_passes(F, parts, passes)) {
             if (++parts > 6) break;
         }
-        if (!engines && !tile_ends() && pair_split(F, pair_buf(), pairs)) {
+        double cost;
+        if (!engines && !tile_ends() && pair_split(F, pair_buf(), pairs, cost)) {
             if (pairs != passes) p.pair_route = true;
             passes = pairs;
             parts = 2;
@@ -1136,18 +1162,11 @@ struct Builder {
             // (up to 16384 points where a compile-time engine exists: one row per CTA)
             if (p.pair_buf && n <= p.max_row_n && pair_choice(static_cast<int>(n), true, false, n, 64, p.pair_buf).P == 0)
                 return add_multipass(n, outer, n, n, src, dst);
-            // Above 4096 points a row and its double buffer leave one CTA per SM: even lengths
-            // without a compile-time engine take two passes of pair tiles (7680 x 1024
-            // 126 -> 64 us, 5000 x 2048 123 -> 108, 4320 x 2048 95 -> 81; odd ones, whose
-            // columns copy 8 bytes at a time, stay: 6561 x 1024 73 us, 97 in two passes).
-            // Complex32 and separated data stay as well (5000 x 838 52 us, 114; 54, 142).
-            if (n > 4096 && n <= kMaxSingleTileC2C && n % 2 == 0 && !p.use_tuned && p.precision == 0 && !tile_ends() &&
-                !find_static_kernel(static_cast<int>(n), IO_C2C)) {
-                std::vector<int> two;
-                if (pair_split(n, kPairBufBytes, two)) {
-                    p.pair_route = true;
-                    return add_multipass(n, outer, n, n, src, dst);
-                }
+            // (even rows without a compile-time engine in two passes of pair tiles)
+            if (n > 4096 && n <= kMaxSingleTileC2C && !p.use_tuned && p.precision == 0 && !tile_ends() &&
+                !find_static_kernel(static_cast<int>(n), IO_C2C) && long_row_in_two(n, outer)) {
+                p.pair_route = true;
+                return add_multipass(n, outer, n, n, src, dst);
             }
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {

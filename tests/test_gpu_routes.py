@@ -130,3 +130,11 @@ def test_short_bluestein(cuda, n, direction):
     for typ in (C2C, R2C, C2R):
         text = _check([n], typ, direction, 333, seed=n)
         assert ("in one kernel" in text) == (2 * n - 1 > 64), text
+
+
+@pytest.mark.parametrize("n,batch,passes", [(4374, 8, 2), (4374, 900, 1), (4410, 8, 2), (4410, 900, 1), (4368, 900, 2),
+                                            (5082, 800, 1), (5000, 800, 2), (7680, 500, 2), (6561, 40, 1)])
+def test_long_rows_without_an_engine(cuda, n, batch, passes):
+    """4097..8192 points: one tile or two passes, by length and size of the data."""
+    text = _check([n], C2C, FWD, batch, seed=n)
+    assert text.startswith(f"steps={passes} "), text
