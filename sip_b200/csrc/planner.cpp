@@ -35,6 +35,7 @@ constexpr int kStaticRowThreads = 128;     // threads per CTA for rows on a comp
 constexpr int kRowSmemTarget = 64 * 1024;  // keep >= 3 CTAs per SM for short rows
 constexpr int kColTile = 16;               // columns per tile: 16 x 8 B = one 128-byte line
 constexpr int kMaxThreads = 512;           // launch bound of the tile kernel (keeps 128 registers/thread)
+constexpr int64_t kL2Bytes = int64_t(126) << 20;
 const int kRadices[] = {16, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
 
 int padded(int i) { return i + (i >> 4); }
@@ -605,6 +606,31 @@ struct Builder {
         return true;
     }
 
+    // Strided FP32 axes: two passes of pair tiles where the axis has no TMA column engine and one
+    // pair tile would keep at most four columns (32-byte row runs, lengths above about 400); the
+    // passes keep 16 and more (us, transposes or column tiles of one transform per thread -> two
+    // passes: 1080 x 1920 x 8 378 -> 180, 1000^2 x 16 322 -> 175, 4096^2 x 1 203 -> 163, 2048^2 r2c
+    // x 4 120 -> 107).  512 and 1024 points with odd strides keep the element-copy tiles of their
+    // engines.  One pass of pair tiles up to 1024 points
+    // * with fewer than 16 columns, which fill no pass's tile (us, one-transform tiles / two passes /
+    //   one: 500 x 7 x 1198 77 / 85 / 61, 729 x 7 x 6575 523 / 673 / 492, 768 x 7 x 48 16 / 17 / 16);
+    // * for odd lengths below 900 with an odd number of columns, whose copies are 8 bytes either way,
+    //   while the data, its intermediate and the result fit L2 (r2c 729^2 x 7 71 / 78 / 68, 625^2 x 10
+    //   92 / 66 / 60; 945 x 65 x 68 84 / 65 / 72).
+    bool strided_axis_in_two(int64_t n, int64_t outer, int64_t inner) const
+    {
+        if (n <= 256 || n > kMaxStridedTile || inner <= 1) return false;
+        const int m = static_cast<int>(n);
+        if ((n <= 1024 && find_static_kernel(m, IO_C2C)) || (col_pipe_has_engine(m) && inner % 2 == 0)) return false;
+        if (pair_columns(m) > 4) return false;
+        if (n > 1024) return true;
+        const bool odd = n % 2 && inner % 2 && n < 900;
+        return inner >= 16 && !(odd && copies_bytes(n * inner, outer) <= kL2Bytes);
+    }
+
+    // the data of a step, its intermediate and the result
+    static int64_t copies_bytes(int64_t points, int64_t outer) { return 3 * int64_t(sizeof(float2)) * points * outer; }
+
     // Rows of 4097..8192 points without a compile-time engine, `outer` of them: two passes of pair
     // tiles, or one tile.  Odd lengths stay in one, since their columns copy 8 bytes at a time
     // (6561 x 1024 73 us, 97 in two passes).  Measured over every even length (13-smooth), us, one
@@ -623,10 +649,9 @@ struct Builder {
         std::vector<int> one, two;
         double cost;
         if (n % 2 || !factor_radices(n, one) || !pair_split(n, kPairBufBytes, two, cost)) return false;
-        constexpr int64_t kL2 = int64_t(126) << 20;
-        const int64_t bytes = 3 * int64_t(sizeof(float2)) * n * outer;
-        if (n >= 6800 || one.size() >= 5 || bytes <= kL2 / 2) return true;
-        if (bytes <= kL2) return cost <= 205 && (two[1] % 2 == 0 || n % 8 == 0 || n >= 4500);
+        const int64_t bytes = copies_bytes(n, outer);
+        if (n >= 6800 || one.size() >= 5 || bytes <= kL2Bytes / 2) return true;
+        if (bytes <= kL2Bytes) return cost <= 205 && (two[1] % 2 == 0 || n % 8 == 0 || n >= 4500);
         return cost <= 190 && n % 16 == 0;
     }
 
@@ -1182,21 +1207,14 @@ struct Builder {
             return false;
         }
         // Tensor-core forms of lengths with the row pipeline: through transposes.
-        // FP32 axes without a TMA column engine whose pair tile would keep at most
-        // four columns (32-byte row runs, lengths above about 400): as two passes of
-        // pair tiles, which keep 16 and more (us, transposes or column tiles of one
-        // transform per thread -> two passes: 1080 x 1920 x 8 378 -> 180, 1000^2 x 16
-        // 322 -> 175, 4096^2 x 1 203 -> 163, 2048^2 r2c x 4 120 -> 107); 512 and 1024
-        // points with odd strides keep the element-copy tiles of their engines.  Vertical 1D plans keep their column
-        // tiles (complex32 data converts in the first and last tile steps).
+        // Vertical 1D plans keep their column tiles (complex32 data converts in the
+        // first and last tile steps).
         if (!in_multipass && p.fft_type != 0x30) {
             TcConfig tcc;
             const int form = tc_form(n);
             if ((form == 1 || form == 2) && tc_rows_config(static_cast<int>(n), tcc))
                 return add_transposed_axis(n, outer, inner, src, dst);
-            if (form == 0 && !p.vertical && n > 256 && n <= kMaxStridedTile && inner > 1 &&
-                !(n <= 1024 && find_static_kernel(static_cast<int>(n), IO_C2C)) &&
-                !(col_pipe_has_engine(static_cast<int>(n)) && inner % 2 == 0) && pair_columns(static_cast<int>(n)) <= 4)
+            if (form == 0 && !p.vertical && strided_axis_in_two(n, outer, inner))
                 return add_multipass(n, outer, n * inner, n * inner, src, dst, inner);
         }
         TileCfg c;

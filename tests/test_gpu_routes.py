@@ -138,3 +138,11 @@ def test_long_rows_without_an_engine(cuda, n, batch, passes):
     """4097..8192 points: one tile or two passes, by length and size of the data."""
     text = _check([n], C2C, FWD, batch, seed=n)
     assert text.startswith(f"steps={passes} "), text
+
+
+@pytest.mark.parametrize("xy,batch,one", [((500, 7), 30, True), ((500, 15), 30, True), ((500, 16), 30, False),
+                                          ((729, 729), 2, True), ((729, 64), 3, False), ((945, 33), 3, False),
+                                          ((1000, 2), 3, True), ((1040, 2), 3, False)])
+def test_strided_axis_in_one_or_two_passes(cuda, xy, batch, one):
+    text = _check(list(xy), C2C, INV, batch, seed=xy[0])
+    assert ("strided x" not in text) == one, text
