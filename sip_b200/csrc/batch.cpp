@@ -274,6 +274,9 @@ struct BatchPlan {
 
 namespace {
 
+// why a set is planned on the one-transform kernels
+const char kNoPairs[] = "a segment has no pair tile, or its workspace would crowd out the data";
+
 std::string build_batch_with(BatchPlan &bp)
 {
     bp.segs.clear();
@@ -283,7 +286,7 @@ std::string build_batch_with(BatchPlan &bp)
     bp.seg_what.clear();
     bp.tables.clear();
     bp.smem = 0;
-    int64_t in_off = 0, ws_off = 0;
+    int64_t in_off = 0, ws_off = 0, pair_ws = 0;  // pair_ws: workspace that only the pair kernel needs
     struct Pending {
         int seg;
         int phase;
@@ -334,7 +337,7 @@ std::string build_batch_with(BatchPlan &bp)
             sg.ntiles = static_cast<int>(s.d.num_tiles);
             sg.fwd = s.forward ? 1 : 0;
             if (bp.pairs) {
-                if (!s.pair) return "a segment has no pair tile";
+                if (!s.pair) return kNoPairs;
                 PairSeg ps{};
                 ps.d = s.pd;
                 ps.in_off = sg.in_off;
@@ -367,6 +370,8 @@ std::string build_batch_with(BatchPlan &bp)
         for (auto &t : p.tables) bp.tables.push_back(t);
         in_off += n * b;
         ws_off += static_cast<int64_t>(ws0 + ws1);
+        if (bp.pairs && n <= kBatchMaxRowN) pair_ws += static_cast<int64_t>(ws0 + ws1);
+        if (pair_ws > spare_copy_bytes(bp.device)) return kNoPairs;
     }
     bp.in_elems = bp.out_elems = in_off;
     bp.ws_bytes = static_cast<size_t>(ws_off);
@@ -414,7 +419,8 @@ std::string build_batch_with(BatchPlan &bp)
 }
 
 // The pair kernel (two transforms per thread) unless a length needs a Bluestein
-// transform; then the one-transform kernels: the compact one (radices up to 10,
+// transform, or rows of 1537..4096 points, which are two passes there, would need
+// workspace for too much data; then the one-transform kernels: the compact one (radices up to 10,
 // three CTAs per SM) when every length factors into them (16 and 12 split),
 // else the one with every radix.
 std::string build_batch(BatchPlan &bp)
@@ -423,7 +429,7 @@ std::string build_batch(BatchPlan &bp)
     bp.pairs = std::all_of(bp.sizes.begin(), bp.sizes.end(), [&](int64_t n) { return n > 1 && factor_radices(n, probe); });
     if (bp.pairs) {
         std::string e = build_batch_with(bp);
-        if (e != "a segment has no pair tile") return e;
+        if (e != kNoPairs) return e;
         bp.pairs = false;
     }
     bp.block = kBatchBlock;

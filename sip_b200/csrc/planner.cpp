@@ -624,6 +624,7 @@ struct Builder {
         if ((n <= 1024 && find_static_kernel(m, IO_C2C)) || (col_pipe_has_engine(m) && inner % 2 == 0)) return false;
         if (pair_columns(m) > 4) return false;
         if (n > 1024) return true;
+        if (copies_bytes(n * inner, outer) / 3 > spare_copy_bytes(device)) return false;  // (no workspace)
         const bool odd = n % 2 && inner % 2 && n < 900;
         return inner >= 16 && !(odd && copies_bytes(n * inner, outer) <= kL2Bytes);
     }
@@ -650,6 +651,7 @@ struct Builder {
         double cost;
         if (n % 2 || !factor_radices(n, one) || !pair_split(n, kPairBufBytes, two, cost)) return false;
         const int64_t bytes = copies_bytes(n, outer);
+        if (bytes / 3 > spare_copy_bytes(device)) return false;  // (no workspace)
         if (n >= 6800 || one.size() >= 5 || bytes <= kL2Bytes / 2) return true;
         if (bytes <= kL2Bytes) return cost <= 205 && (two[1] % 2 == 0 || n % 8 == 0 || n >= 4500);
         return cost <= 190 && n % 16 == 0;

@@ -155,6 +155,7 @@ namespace {
 std::mutex g_dev_mu;
 std::map<int, int *> g_err_words;
 std::map<int, int> g_sms;
+std::map<int, int64_t> g_spare;
 }  // namespace
 
 int *device_error_word(int device)
@@ -208,6 +209,19 @@ int sm_count(int device)
     }
     g_sms[device] = n;
     return n;
+}
+
+int64_t spare_copy_bytes(int device)
+{
+    std::lock_guard<std::mutex> lock(g_dev_mu);
+    auto it = g_spare.find(device);
+    if (it != g_spare.end()) return it->second;
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return g_spare[device] = static_cast<int64_t>(total / 4);
 }
 
 std::string complex32_steps(const Plan &p, std::vector<Step> &out)

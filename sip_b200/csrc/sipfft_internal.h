@@ -137,6 +137,9 @@ int *device_error_word(int device);
 void set_last_error(const std::string &msg);
 const std::string &last_error();
 int sm_count(int device);
+// Largest copy of the data that a plan takes as workspace where a route without it exists:
+// a quarter of the (current) device's memory, so that input, output and workspace fit.
+int64_t spare_copy_bytes(int device);
 // R2C post-twiddle / C2R pre-twiddle of the multi-pass (large-N) plans.
 cudaError_t launch_r2c_post(const float2 *z, float2 *x, int64_t rows, int64_t m, int64_t zdist, int64_t xdist,
                             const float2 *tw_lo, const float2 *tw_hi, int log2l, bool forward, cudaStream_t st);

@@ -146,3 +146,30 @@ def test_long_rows_without_an_engine(cuda, n, batch, passes):
 def test_strided_axis_in_one_or_two_passes(cuda, xy, batch, one):
     text = _check(list(xy), C2C, INV, batch, seed=xy[0])
     assert ("strided x" not in text) == one, text
+
+
+def test_data_too_large_to_hold_once_more(cuda):
+    """Planning only: routes that need a copy of the data as workspace where another route
+    does not are taken while input, output and that copy fit the device."""
+    import torch
+
+    quarter = torch.cuda.mem_get_info()[1] // 4
+    for sizes in ([600, 600], [5000]):
+        points = int(np.prod(sizes))
+        for batch, fits in ((quarter // (8 * points), True), (quarter // (8 * points) + 1, False)):
+            h = fft.asdFftCreate()
+            st = (fft.asdFftMakePlan1D(h, sizes[0], C2C, FWD, batch) if len(sizes) == 1 else
+                  fft.asdFftMakePlan2D(h, *sizes, C2C, FWD, batch))
+            assert st == fft.ACL_SUCCESS
+            assert (fft.asdFftGetWorkspaceSize(h)[1] > 0) == fits, fft.describe_plan(h)
+            fft.asdFftDestroy(h)
+    import ctypes
+
+    lib = fft.load_library()
+    for batch, fits in ((quarter // (8 * 2000), True), (quarter // (8 * 2000) + 1, False)):
+        h, need = ctypes.c_void_p(), ctypes.c_size_t()
+        one = lambda v: (ctypes.c_int64 * 1)(v)
+        assert lib.asdFftBatchPlanCreate(ctypes.byref(h), one(2000), one(batch), 1, FWD, None) == fft.ACL_SUCCESS
+        assert lib.asdFftBatchGetWorkspaceSize(h, ctypes.byref(need)) == fft.ACL_SUCCESS
+        assert (need.value > 0) == fits
+        lib.asdFftBatchPlanDestroy(h)
