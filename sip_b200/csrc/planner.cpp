@@ -553,18 +553,25 @@ struct Builder {
             max_pairs /= 2;
         PairDesc q{};
         std::vector<int> radices;
-        int P = static_cast<int>(max_pairs);
+        const int most_pairs = static_cast<int>(max_pairs);
+        int P = 0;
+        auto shaped = [&](int first) {
+            const int S = static_cast<int>(radices.size());
+            for (P = first; P >= 1 && S > 0; P /= 2)
+                if (pair_shape(q, d.n, radices.data(), S, rows, runs, in_dist, P, pair_buf())) return true;
+            return false;
+        };
+        bool ok = false;
         if (tuned) {
             radices = tuned->radices;
-            if (tuned->row_threads > 0 && tuned->row_threads <= 128) P = std::min(P, 4);
-        } else {
-            const PairChoice c = pair_choice(d.n, rows, runs, in_dist, P, pair_buf());
-            radices = c.radices;
-            P = c.P;
+            ok = shaped(tuned->row_threads > 0 && tuned->row_threads <= 128 ? std::min(most_pairs, 4) : most_pairs);
         }
-        while (P >= 1 && !radices.empty() && !pair_shape(q, d.n, radices.data(), static_cast<int>(radices.size()), rows, runs, in_dist, P, pair_buf()))
-            P /= 2;
-        if (P < 1 || radices.empty()) return true;
+        if (!ok) {  // (a tuned sequence may have no pair tile: 1440 = 12 x 12 x 10 has more butterflies than threads)
+            const PairChoice c = pair_choice(d.n, rows, runs, in_dist, most_pairs, pair_buf());
+            radices = c.radices;
+            ok = shaped(c.P);
+        }
+        if (!ok) return true;
         const int64_t per_outer = (d.n_cols + 2 * q.P - 1) / (2 * q.P), tiles = per_outer * d.n_outer;
         if (tiles >= most) return true;
         const int per_sm = kernel_blocks_per_sm(pair_kernel_fn(s.forward), kPairThreads, pair_smem(q.buf_words));

@@ -173,3 +173,39 @@ def test_data_too_large_to_hold_once_more(cuda):
         assert lib.asdFftBatchGetWorkspaceSize(h, ctypes.byref(need)) == fft.ACL_SUCCESS
         assert (need.value > 0) == fits
         lib.asdFftBatchPlanDestroy(h)
+
+
+def test_tuned_sequence_without_a_pair_tile(cuda, tmp_path):
+    """A cache entry whose radices have no pair tile does not take the whole uneven batch to
+    the one-transform kernel: the planner's own radices stand in."""
+    import json
+
+    import torch
+
+    path = str(tmp_path / "tune.jsonl")
+    entries = {1440: [12, 12, 10], 1296: [9, 12, 12], 1536: [8, 16, 12], 500: [10, 5, 10]}
+    with open(path, "w") as f:
+        for n, r in entries.items():
+            f.write(json.dumps({"gpu": torch.cuda.get_device_name(0), "type": "c2c", "precision": "fp32", "n": n,
+                                "radices": r, "maxe": 16, "row_threads": 256, "us": 1.0, "plan_us": 0}) + "\n")
+    groups = [(n, 7) for n in entries]
+    for direction in (FWD, INV):
+        plan = fft.BatchPlan(groups, direction, path)
+        text = plan.describe()
+        assert "kernel=pairs" in text, text
+        assert "n=500 tiles" in text and "radices=10x5x10" in text, text  # (an entry that fits is used)
+        rng = np.random.default_rng(5)
+        x = (rng.uniform(-1, 1, plan.total) + 1j * rng.uniform(-1, 1, plan.total)).astype(np.complex64)
+        y = torch.zeros(plan.total, dtype=torch.complex64, device="cuda")
+        plan(torch.from_numpy(x).cuda(), y)
+        plan.synchronize()
+        for (n, b), off in zip(plan.groups, plan.offsets):
+            got = y[off:off + n * b].cpu().numpy().reshape(b, n)
+            assert oracle.rel_l2(got, oracle.c2c(x[off:off + n * b].reshape(b, n), direction == FWD)) <= oracle.tolerance(n)
+        plan.close()
+    # (the choices stay with the process: empty ones give the lengths back to the planner)
+    with open(path, "w") as f:
+        for n in entries:
+            f.write(json.dumps({"gpu": torch.cuda.get_device_name(0), "type": "c2c", "precision": "fp32", "n": n,
+                                "radices": [], "maxe": 0, "row_threads": 0, "us": 0, "plan_us": 0}) + "\n")
+    assert fft.tune_cache_load(path) == len(entries)
