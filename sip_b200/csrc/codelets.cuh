@@ -69,6 +69,15 @@ SIPFFT_HD float2 cmul(float2 a, float2 b)
 {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
+// The product of the roots of unity 1 + l and 1 + h, given without their one, l of a
+// small angle: values round at their own size and the smallest are added first, so that
+// the product carries little more than its own rounding (two rounded roots multiplied:
+// three roundings).
+SIPFFT_HD float2 root_product(float2 l, float2 h)
+{
+    const float re = l.x + fmaf(l.x, h.x, -l.y * h.y), im = l.y + fmaf(l.x, h.y, l.y * h.x);
+    return make_float2(1.f + (h.x + re), h.y + im);
+}
 SIPFFT_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 SIPFFT_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 SIPFFT_HD float2 cneg(float2 a) { return neg2(a); }

@@ -383,13 +383,18 @@ __global__ void __launch_bounds__(kBatchBlock, COMPACT ? 3 : 2)
 // t[m] = exp(-2 pi i * ((m * mult) mod denom) / denom), evaluated in FP64 and
 // rounded once to FP32 (the reference builds its tables the same way on the
 // host: core/fft/fftcore/fft_core_common_func.cpp:214-232).
-__global__ void twiddle_kernel(float2 *t, int64_t count, int64_t denom, int64_t mult)
+// less_one: minus 1, as -2 sin^2 of half the angle.
+__global__ void twiddle_kernel(float2 *t, int64_t count, int64_t denom, int64_t mult, bool less_one)
 {
     for (int64_t m = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; m < count;
          m += int64_t(gridDim.x) * blockDim.x) {
         const int64_t idx = (m * mult) % denom;
         double s, c;
         sincospi(2.0 * static_cast<double>(idx) / static_cast<double>(denom), &s, &c);
+        if (less_one) {
+            const double h = sinpi(static_cast<double>(idx) / static_cast<double>(denom));
+            c = -2.0 * h * h;
+        }
         t[m] = make_float2(static_cast<float>(c), static_cast<float>(-s));
     }
 }
@@ -553,13 +558,13 @@ cudaError_t launch_batch(int grid, int block, size_t smem, const BatchSeg *segs,
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, st);
 }
 
-cudaError_t fill_twiddles(float2 *t, int64_t count, int64_t denom, int64_t mult, cudaStream_t st)
+cudaError_t fill_twiddles(float2 *t, int64_t count, int64_t denom, int64_t mult, cudaStream_t st, bool less_one)
 {
     if (count <= 0) return cudaSuccess;
     const int block = 256;
     int64_t grid = (count + block - 1) / block;
     if (grid > 4096) grid = 4096;
-    twiddle_kernel<<<static_cast<int>(grid), block, 0, st>>>(t, count, denom, mult);
+    twiddle_kernel<<<static_cast<int>(grid), block, 0, st>>>(t, count, denom, mult, less_one);
     return cudaGetLastError();
 }
 

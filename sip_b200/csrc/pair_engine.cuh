@@ -47,18 +47,20 @@ struct PairTile {
 // complex values, [element][P pairs]).  A multi-pass step multiplies element
 // e = j + r N/R0 of Stockham column k by W^(e k) = t1[j][k] t2[r][k]: both
 // tables are contiguous in k, adjacent columns read adjacent entries, and the
-// product has one rounding more than a single table, as the two-level table
-// lookup has.  Against that lookup (two gathers at computed indices for every
-// element of every column) it needs no index arithmetic per element.
-// The two-level table of the same twiddles (t1 rows where t1 is not built).
+// product of two rounded entries is as exact as the two-level table lookup (rms
+// 3.3e-8 either way).  Against that lookup (two gathers at computed indices for
+// every element of every column) it needs no index arithmetic per element.
+// Where t1 is not built (more than 8 MB) its entries come from two short tables
+// of roots less one (root_product: 2.1e-8; a third rounded factor would make the
+// product 4.0e-8).
 struct PassTable2 {
-    const float2 *lo, *hi;
+    const float2 *lo, *hi;  // exp(-2 pi i m / F) - 1, m < 2^log2l, and for multiples of 2^log2l
     int log2l;
     uint32_t step;
     __device__ __forceinline__ float2 at(int e, uint32_t k) const
     {
         const uint32_t m = static_cast<uint32_t>(e) * k * step;
-        return cmul(__ldg(lo + (m & ((1u << log2l) - 1u))), __ldg(hi + (m >> log2l)));
+        return root_product(__ldg(lo + (m & ((1u << log2l) - 1u))), __ldg(hi + (m >> log2l)));
     }
 };
 

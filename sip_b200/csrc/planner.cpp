@@ -291,21 +291,21 @@ struct Builder {
     // the first and last step run on the generic tile kernel (Plan::tile_ends)
     bool tile_ends() const { return p.tile_ends || p.fft_type == 0x30; }
 
-    const float2 *table(int64_t count, int64_t denom, int64_t mult = 1)
+    const float2 *table(int64_t count, int64_t denom, int64_t mult = 1, bool less_one = false)
     {
-        TablePtr t = get_table(count, denom, mult, device, &err);
+        TablePtr t = get_table(count, denom, mult, device, &err, less_one);
         if (!t) return nullptr;
         p.tables.push_back(t);
         return t->ptr;
     }
 
-    // two-level table for W_F^m, m < F: lo[m & (L-1)] * hi[m >> log2 L]
-    bool table2(int64_t F, const float2 *&lo, const float2 *&hi, int &log2l)
+    // two-level table for W_F^m, m < F: lo[m & (L-1)] * hi[m >> log2 L] (less_one: root_product)
+    bool table2(int64_t F, const float2 *&lo, const float2 *&hi, int &log2l, bool less_one = false)
     {
         log2l = std::max(1, (ilog2_ceil(F) + 1) / 2);
         const int64_t L = int64_t(1) << log2l;
-        lo = table(L, F, 1);
-        hi = table((F + L - 1) / L, F, L);
+        lo = table(L, F, 1, less_one);
+        hi = table((F + L - 1) / L, F, L, less_one);
         return lo && hi;
     }
 
@@ -665,21 +665,25 @@ struct Builder {
     }
 
     // Inter-pass twiddle tables of a kernel of two columns per thread whose
-    // first radix is r0: t1 up to 8 MB (beyond it the rows of t1 come from the
-    // two-level table), t2 always.
-    bool pass_tables(const TileDesc &d, int r0, const float2 *&t1, const float2 *&t2)
+    // first radix is r0, with descriptor `q`: t1 up to 8 MB (beyond it its entries
+    // come from the two-level table of roots less one, which the descriptor then
+    // holds), t2 always: r0 / n of the size of one transform, 32 MB of 2^27 points' 1 GB.
+    template <class Desc>
+    bool pass_tables(const TileDesc &d, int r0, Desc &q)
     {
         const int64_t rows = d.n / r0;
         if (rows * d.g_ns <= int64_t(1) << 20) {
             TablePtr t = get_outer_table(rows, d.g_ns, d.g_ns * d.n, device, &err);
             if (!t) return false;
             p.tables.push_back(t);
-            t1 = t->ptr;
+            q.g_t1 = t->ptr;
+        } else if (!table2(d.g_step * d.g_ns * d.n, q.g_lo, q.g_hi, q.g_log2l, true)) {
+            return false;
         }
         TablePtr t = get_outer_table(r0, d.g_ns, d.g_ns * r0, device, &err);
         if (!t) return false;
         p.tables.push_back(t);
-        t2 = t->ptr;
+        q.g_t2 = t->ptr;
         return true;
     }
 
@@ -692,23 +696,17 @@ struct Builder {
             c.g_ns = d.g_ns;
             c.g_div = d.g_div;
             c.g_step = d.g_step;
-            c.g_lo = d.g_lo;
-            c.g_hi = d.g_hi;
-            c.g_log2l = d.g_log2l;
             c.dv_gdiv = fast_div(d.g_div);
             c.dv_gns = fast_div(d.g_ns);
-            if (d.g_twiddle && !pass_tables(d, c.radix[0], c.g_t1, c.g_t2)) return false;
+            if (d.g_twiddle && !pass_tables(d, c.radix[0], c)) return false;
         }
         if (s.pair) {
             PairDesc &q = s.pd;
             q.g_twiddle = d.g_twiddle;
             q.g_step = d.g_step;
-            q.g_lo = d.g_lo;
-            q.g_hi = d.g_hi;
-            q.g_log2l = d.g_log2l;
             q.dv_gdiv = fast_div(d.g_div);
             q.dv_gns = fast_div(d.g_ns);
-            if (d.g_twiddle && !pass_tables(d, q.st[0].R, q.g_t1, q.g_t2)) return false;
+            if (d.g_twiddle && !pass_tables(d, q.st[0].R, q)) return false;
         }
         return true;
     }

@@ -29,13 +29,13 @@ DeviceTable::~DeviceTable()
 
 namespace {
 std::mutex g_table_mu;
-std::map<std::tuple<int, int64_t, int64_t, int64_t>, std::weak_ptr<DeviceTable>> g_tables;
+std::map<std::tuple<int, int64_t, int64_t, int64_t, bool>, std::weak_ptr<DeviceTable>> g_tables;
 }  // namespace
 
-TablePtr get_table(int64_t count, int64_t denom, int64_t mult, int device, std::string *err)
+TablePtr get_table(int64_t count, int64_t denom, int64_t mult, int device, std::string *err, bool less_one)
 {
     std::lock_guard<std::mutex> lock(g_table_mu);
-    auto key = std::make_tuple(device, count, denom, mult);
+    auto key = std::make_tuple(device, count, denom, mult, less_one);
     auto it = g_tables.find(key);
     if (it != g_tables.end()) {
         if (TablePtr t = it->second.lock()) return t;
@@ -44,7 +44,7 @@ TablePtr get_table(int64_t count, int64_t denom, int64_t mult, int device, std::
     t->count = count;
     t->device = device;
     cudaError_t e = cudaMalloc(&t->ptr, sizeof(float2) * static_cast<size_t>(count));
-    if (e == cudaSuccess) e = fill_twiddles(t->ptr, count, denom, mult, 0);
+    if (e == cudaSuccess) e = fill_twiddles(t->ptr, count, denom, mult, 0, less_one);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) {
         if (err) *err = std::string("twiddle table: ") + cudaGetErrorString(e);

@@ -23,7 +23,8 @@ cudaError_t launch_tile(const TileDesc &d, int maxe, bool forward, int grid, cud
 // Persistent double-buffered C2C tile kernel (cp.async prefetch of the next tile).
 const void *tile_db_kernel_fn(int maxe, bool forward);
 cudaError_t launch_tile_db(const TileDesc &d, int maxe, bool forward, int grid, cudaStream_t st);
-cudaError_t fill_twiddles(float2 *t, int64_t count, int64_t denom, int64_t mult, cudaStream_t st);
+cudaError_t fill_twiddles(float2 *t, int64_t count, int64_t denom, int64_t mult, cudaStream_t st,
+                          bool less_one = false);
 cudaError_t fill_chirp(float2 *t, int64_t n_len, bool forward, cudaStream_t st);
 cudaError_t fill_bluestein_b(float2 *b, const float2 *chirp, int64_t n_len, int64_t m_len, cudaStream_t st);
 cudaError_t scale_table(float2 *b, int64_t count, float s, cudaStream_t st);
@@ -170,7 +171,8 @@ struct DeviceTable {
 };
 using TablePtr = std::shared_ptr<DeviceTable>;
 // t[m] = exp(-2 pi i (m*mult mod denom) / denom), m < count
-TablePtr get_table(int64_t count, int64_t denom, int64_t mult, int device, std::string *err);
+// exp(-2 pi i m mult / denom), m < count; less_one: minus 1
+TablePtr get_table(int64_t count, int64_t denom, int64_t mult, int device, std::string *err, bool less_one = false);
 // per-stage twiddle tables of a static kernel's radix sequence
 TablePtr get_stage_table(const StaticKernel &k, int device, std::string *err);
 // per-stage twiddle tables of any radix sequence: stage s >= 1 holds

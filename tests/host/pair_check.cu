@@ -10,6 +10,7 @@
 #include <cstring>
 #include <vector>
 
+#include "codelets.cuh"
 #include "pair_tile.cuh"
 
 using namespace sipfft;
@@ -118,10 +119,46 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
     return true;
 }
 
+// Inter-pass twiddles W_F^(e k), e = j + r n / r0, in FP32: the rms error of t1 t2 with t1 from
+// the tables of roots less one is not above that of one two-level lookup (two rounded factors).
+static bool twiddles(int64_t F, int n, int r0)
+{
+    auto root = [](int64_t m, int64_t d) {
+        const double t = 2 * M_PI * double(m % d) / double(d);
+        return make_float2(float(std::cos(t)), float(-std::sin(t)));
+    };
+    auto less_one = [](int64_t m, int64_t d) {
+        const double t = M_PI * double(m % d) / double(d), s = std::sin(t);
+        return make_float2(float(-2 * s * s), float(-std::sin(2 * t)));
+    };
+    int log2l = 1;
+    while ((int64_t(1) << (2 * log2l)) < F) log2l++;
+    const int64_t L = int64_t(1) << log2l, ns = F / n;
+    double lookup = 0, product = 0;
+    uint64_t seed = 12345;
+    auto draw = [&](int64_t below) {
+        seed = seed * 6364136223846793005ull + 1442695040888963407ull;
+        return int64_t((seed >> 33) % uint64_t(below));
+    };
+    for (int i = 0; i < 200000; i++) {
+        const int64_t k = draw(ns), j = draw(n / r0), r = draw(r0), m = (j + r * (n / r0)) * k % F, u = j * k;
+        const cd exact = std::polar(1.0, -2 * M_PI * double(m) / double(F));
+        auto off = [&](float2 w) { return std::norm(cd(w.x, w.y) - exact); };
+        const float2 t2 = root(r * k * (n / r0), F);
+        lookup += off(cmul(root(m % L, F), root(m / L * L, F)));
+        product += off(cmul(root_product(less_one(u % L, F), less_one(u / L * L, F)), t2));
+    }
+    if (product <= lookup * 1.02) return true;  // (2 %: the spread of 200000 draws)
+    std::printf("FAILED twiddles F=%lld n=%d r0=%d: lookup %.3g product %.3g\n", (long long)F, n, r0,
+                std::sqrt(lookup / 2e5), std::sqrt(product / 2e5));
+    return false;
+}
+
 int main()
 {
     int shapes = 0;
     bool ok = true;
+    ok = twiddles(1 << 25, 256, 16) && twiddles(1 << 27, 512, 16) && twiddles(15625 * 2048, 250, 10) && ok;
     std::vector<int> lengths;
     for (int n = 2; n <= 100; n++) lengths.push_back(n);
     for (int n : {210, 225, 240, 243, 250, 252, 256, 300, 343, 375, 400, 441, 480, 512, 540, 625, 720, 768, 960, 1000,

@@ -1,6 +1,7 @@
 """CPU: the index arithmetic of the pair tiles (two transforms per thread) is walked
 element by element for every tile shape of a range of lengths: bounds of the
-shared-memory words, every butterfly once, and the transform itself."""
+shared-memory words, every butterfly once, and the transform itself; and the rounding
+of the inter-pass twiddles."""
 import os
 import shutil
 import subprocess
