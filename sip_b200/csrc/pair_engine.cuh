@@ -78,12 +78,10 @@ struct PassTwiddle {
             return pair_of(__ldg(p), __ldg(p - k0 + k1));
         }
     }
-    // v[r] *= W^((j + r NBF) k) of both columns, r < R
+    // v[r] *= w0 t2[r][k] of both columns, r < R: w0 = W^(j k), the product W^((j + r NBF) k)
     template <int R, bool FWD, bool ADJACENT>
-    __device__ __forceinline__ void apply(cpx2 *v, int j, const PassTable2 &two) const
+    __device__ __forceinline__ void apply(cpx2 *v, cpx2 w0) const
     {
-        const cpx2 w0 = t1 ? at<ADJACENT>(t1, j)
-                           : pair_of(two.at(j, k0), two.at(j, k1));
         v[0] = cmul(v[0], dir<FWD>(w0));
 #pragma unroll
         for (int r = 1; r < R; r++) v[r] = cmul(v[r], dir<FWD>(cmul(w0, at<ADJACENT>(t2, r))));
@@ -107,10 +105,13 @@ __device__ __forceinline__ void pair_stage0(cpx2 *v, const float4 *tile, int lan
 #pragma unroll
     for (int b = 0; b < NB; b++) {
         if (tw.t2) {
+            const int j = lane + b * T;
             if (tw.k1 == tw.k0 + 1 && ((tw.k0 | tw.ns) & 1) == 0)
-                tw.template apply<R, FWD, true>(v + b * R, lane + b * T, two);
+                tw.template apply<R, FWD, true>(
+                    v + b * R, tw.t1 ? tw.at<true>(tw.t1, j) : pair_of(two.at(j, tw.k0), two.at(j, tw.k1)));
             else
-                tw.template apply<R, FWD, false>(v + b * R, lane + b * T, two);
+                tw.template apply<R, FWD, false>(
+                    v + b * R, tw.t1 ? tw.at<false>(tw.t1, j) : pair_of(two.at(j, tw.k0), two.at(j, tw.k1)));
         }
         dft<R, FWD>(v + b * R);
     }

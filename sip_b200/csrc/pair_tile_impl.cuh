@@ -113,7 +113,11 @@ __device__ __forceinline__ float4 word_of(cpx2 v) { return make_float4(v.re.x, v
 // Where a stage reads, and how the threads walk the tile: rows with the
 // elements fastest, columns with the pairs fastest; a work tile either way (the
 // last stage of columns whose outputs are contiguous takes the elements fastest).
-enum PairSource { kPairRows = 0, kPairCols = 1, kPairColsTwiddled = 2, kPairWorkE = 3, kPairWorkP = 4 };
+// (Twiddled columns of the longest rows, whose t1 is not built, have stages of their own: the
+// lookup's registers slowed the others by up to 12 %, 96000 x 43 40 -> 45 us.)
+enum PairSource {
+    kPairRows = 0, kPairCols = 1, kPairColsTwiddled = 2, kPairColsTwiddled2 = 3, kPairWorkE = 4, kPairWorkP = 5
+};
 
 // One stage of radix R: reads the staged tile (rows, columns, columns with the
 // inter-pass twiddles of a multi-pass step) or the work tile, writes the work
@@ -124,7 +128,8 @@ template <int R, PairSource SRC, bool FWD>
 __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTileState s)
 {
     constexpr int NB = pair_nb(R);
-    constexpr bool FIRST = SRC <= kPairColsTwiddled;
+    constexpr bool TWIDDLED = SRC == kPairColsTwiddled || SRC == kPairColsTwiddled2;
+    constexpr bool FIRST = SRC <= kPairColsTwiddled2;
     constexpr bool E = SRC == kPairRows || SRC == kPairWorkE;  // elements fastest
     const PairDesc &d = pair_slot(s.slot).d;
     const PairStage &t = d.st[stage];
@@ -154,10 +159,11 @@ __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTil
     auto block = [&](int j) { return FIRST ? j : static_cast<int>(__umulhi(static_cast<uint32_t>(j), ns_m)); };  // j div ns
     PassTwiddle tw{};
     PassTable2 two{};
-    if constexpr (SRC == kPairColsTwiddled) {
+    if constexpr (TWIDDLED) {
         const uint32_t c = s.c0 + 2 * p0;
         tw = PassTwiddle{d.g_t1, d.g_t2, d.dv_gns.d, d.dv_gns.mod(d.dv_gdiv.div(c)), d.dv_gns.mod(d.dv_gdiv.div(c + 1))};
-        two = PassTable2{d.g_lo, d.g_hi, d.g_log2l, static_cast<uint32_t>(d.g_step)};
+        if constexpr (SRC == kPairColsTwiddled2)
+            two = PassTable2{d.g_lo, d.g_hi, d.g_log2l, static_cast<uint32_t>(d.g_step)};
     }
 #pragma unroll
     for (int b = 0; b < NB; b++) {
@@ -177,7 +183,10 @@ __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTil
                 const float4 u = w[r * step];
                 v[b * R + r] = pair_of(make_float2(u.x, u.y), make_float2(u.z, u.w));
             }
-            if constexpr (SRC == kPairColsTwiddled) tw.template apply<R, FWD, false>(v + b * R, j, two);
+            if constexpr (SRC == kPairColsTwiddled)
+                tw.template apply<R, FWD, false>(v + b * R, tw.at<false>(tw.t1, j));
+            if constexpr (SRC == kPairColsTwiddled2)
+                tw.template apply<R, FWD, false>(v + b * R, pair_of(two.at(j, tw.k0), two.at(j, tw.k1)));
         } else {
             const int q = block(j);
             const float4 *w = pair_smem + s.buf + pair_gather_at(SP, SE, t.gpad, p, j, q);
@@ -384,8 +393,10 @@ __device__ __forceinline__ void pair_tile(int slot, int buf, const void *in, voi
     }
     if (d.rows)
         pair_any<kPairRows, FWD>(d.st[0].R, 0, S == 1 && direct, s);
-    else if (d.g_twiddle)
+    else if (d.g_twiddle && d.g_t1)
         pair_any<kPairColsTwiddled, FWD>(d.st[0].R, 0, S == 1, s);
+    else if (d.g_twiddle)
+        pair_any<kPairColsTwiddled2, FWD>(d.st[0].R, 0, S == 1, s);
     else
         pair_any<kPairCols, FWD>(d.st[0].R, 0, S == 1, s);
 #pragma unroll 1
