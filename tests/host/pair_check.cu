@@ -154,10 +154,58 @@ static bool twiddles(int64_t F, int n, int r0)
     return false;
 }
 
+// Relative rms error of the radix-R codelet on two transforms (index 0) and on one (index 1).
+template <int R, bool FWD>
+static void codelet_errors(double (&e)[2])
+{
+    double err[2] = {}, ref = 0;
+    uint32_t seed = 7;
+    auto draw = [&] { return float(((seed = seed * 1664525u + 1013904223u) >> 8) / 8388608.0 - 1.0); };
+    for (int t = 0; t < 4000; t++) {
+        float2 one[R];
+        cpx2 two[R];
+        cd x[R];
+        for (int i = 0; i < R; i++) {
+            one[i].x = draw();
+            one[i].y = draw();
+            x[i] = cd(one[i].x, one[i].y);
+            two[i] = pair_of(make_float2(draw(), draw()), one[i]);
+        }
+        dft<R, FWD>(one);
+        dft<R, FWD>(two);
+        for (int k = 0; k < R; k++) {
+            cd y = 0;
+            for (int j = 0; j < R; j++) y += x[j] * std::polar(1.0, (FWD ? -2 : 2) * M_PI * ((j * k) % R) / R);
+            const float2 s = second_of(two[k]);
+            err[0] += std::norm(cd(s.x, s.y) - y);
+            err[1] += std::norm(cd(one[k].x, one[k].y) - y);
+            ref += std::norm(y);
+        }
+    }
+    for (int i = 0; i < 2; i++) e[i] = std::sqrt(err[i] / ref);
+}
+
+// Primes and powers of two: the same operations.  Composites: no twiddles on two transforms, and
+// fewer roundings (each input passes the products of one twiddle less: at least 4 % of the error).
+template <int R>
+static bool codelets()
+{
+    double f[2], b[2];
+    codelet_errors<R, true>(f);
+    codelet_errors<R, false>(b);
+    const bool composite = R == 6 || R == 10 || R == 12 || R == 14 || R == 15;
+    const bool ok = composite ? f[0] < 0.96 * f[1] && b[0] < 0.96 * b[1] : f[0] == f[1] && b[0] == b[1];
+    if (!ok) std::printf("FAILED radix %d: two %.3g %.3g one %.3g %.3g\n", R, f[0], b[0], f[1], b[1]);
+    return ok;
+}
+
 int main()
 {
     int shapes = 0;
     bool ok = true;
+    ok = codelets<2>() && codelets<3>() && codelets<4>() && codelets<5>() && codelets<6>() && codelets<7>() &&
+         codelets<8>() && codelets<9>() && codelets<10>() && codelets<11>() && codelets<12>() && codelets<13>() &&
+         codelets<14>() && codelets<15>() && codelets<16>();
     ok = twiddles(1 << 25, 256, 16) && twiddles(1 << 27, 512, 16) && twiddles(15625 * 2048, 250, 10) && ok;
     std::vector<int> lengths;
     for (int n = 2; n <= 100; n++) lengths.push_back(n);
