@@ -528,16 +528,22 @@ struct Builder {
                 return true;
             in_dist = d.in_a.cstride;
             out_dist = d.out_a.cstride;
-            // Rows of a few points: a tile's fixed work is spread over too little, and the
+            // Many rows of a few points: a tile's fixed work is spread over too little, and the
             // one-transform tile kernel is faster (4 M points, us, pair tiles -> tile kernel: c2c
-            // 2 points 51 -> 31, 5 28 -> 23, 12 31 -> 26, 13 26 -> 25, 14 equal; r2c 8 20 -> 15).
-            if (d.n < 14 && !p.use_tuned) return true;
+            // 2 points 51 -> 31, 5 28 -> 23, 12 31 -> 26, 13 26 -> 25, 14 27 <- 31; c2r 22 20 -> 18;
+            // r2c 8 20 -> 15, 10 16 -> 15, but 14 12 <- 15 and 22 10 <- 16).  Few rows leave the SMs
+            // idle either way, and the pair tile's chain is shorter (8 points, device time: 5000
+            // rows 2.8 <- 3.4, 30000 4.3 -> 3.8; 13 points 2.9 <- 4.1, 4.7 <- 4.8).
+            if (d.n < (d.io == IO_R2C_PACKED ? 6 : 14) && d.n_cols > 16384 && !p.use_tuned) return true;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
-        } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32)) {
+        } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32) &&
+                   d.n_outer > (d.n >= 9 ? 8 : 4) * int64_t(sm_count(device))) {
             // Few short columns (one tile per outer index, of a few hundred points at most): the
-            // one-transform tiles put more CTAs on an SM (4 M points, us, pair tiles / those: 8 x 8
-            // 1.95, 16 x 12 1.44, 30 x 9 1.43, 20 x 5 2.0; 36 x 9 1.0, 16 x 24 0.91, 8 x 33 0.90).
+            // one-transform tiles put more CTAs on an SM (4 M points, time of pair tiles / of those:
+            // 8 x 8 1.95, 16 x 12 1.44, 30 x 9 1.43, 20 x 5 2.0; 36 x 9 1.0, 16 x 24 0.91, 8 x 33
+            // 0.90).  Up to one wave of pair tiles (two from 9 points on) those are faster (both axes,
+            // device time, us: 8 x 8 x 256 6.0 / 7.1, x 1024 9.7 / 8.7; 30 x 9 x 1024 12 / 15).
             return true;
         } else if (d.io != IO_C2C || d.in_a.cstride != 1 || d.in_a.cblock != 0 || d.out_a.cblock >= most) {
             return true;
@@ -986,11 +992,13 @@ struct Builder {
         }
         // In one kernel where the convolution fits a pair tile, with the cheapest
         // length among a few times powers of two (planar data and uneven batches
-        // keep tile steps).  Convolutions of up to 64 points keep them too: the row by
-        // row element-wise passes cost more than the saved intermediate (4 M points, us,
-        // one kernel / two launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317).
+        // keep tile steps).  Convolutions of up to 64 points keep them too, but for a few
+        // rows: a tile of 32 rows goes through its element-wise passes row by row, which
+        // costs more than the saved intermediate (4 M points, us, one kernel / two
+        // launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317; c2c 17 x 1 4.6 / 18,
+        // c2r 17 x 64 25 / 21).
         PairChoice fused;
-        if (p.fft_type != 0x30 && !p.use_tuned && 2 * n - 1 > 64 && rows < (int64_t(1) << 31)) {
+        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= 16) && rows < (int64_t(1) << 31)) {
             const int64_t pow2 = m;
             double best = 1e30;
             for (int64_t f : {1, 3, 5, 7, 9, 15}) {

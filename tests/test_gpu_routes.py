@@ -102,34 +102,40 @@ def _check(sizes, typ, direction, batch, seed, vertical=False):
 @pytest.mark.parametrize("n", list(range(2, 17)))
 @pytest.mark.parametrize("direction", [FWD, INV])
 def test_short_rows(cuda, n, direction):
-    """Rows of fewer than 14 points (packed points of real rows) on the tile kernel."""
+    """Many rows of fewer than 14 points (packed points of C2R rows; of R2C rows fewer than 6)
+    on the tile kernel."""
     for typ, k in ((C2C, n), (R2C, 2 * n), (C2R, 2 * n)):
-        text = _check([k], typ, direction, 1031, seed=n)
-        assert ("[pair tiles]" in text) == (n >= 14 and "static" not in text), text
+        for batch in (1031, 16385):
+            text = _check([k], typ, direction, batch, seed=n)
+            pairs = n >= (6 if typ == R2C else 14) or batch < 16385
+            assert ("[pair tiles]" in text) == (pairs and "static" not in text), text
 
 
 @pytest.mark.parametrize("xy", [(3, 7), (8, 8), (8, 33), (9, 16), (9, 17), (16, 12), (16, 24), (30, 9), (32, 16), (33, 9),
                                 (36, 2)])
 @pytest.mark.parametrize("direction", [FWD, INV])
 def test_short_narrow_columns(cuda, xy, direction):
-    """Columns of up to 32 points, at most 16 of them (32 below 9 points), on the tile kernel."""
+    """Columns of up to 32 points, at most 16 of them (32 below 9 points), on the tile kernel
+    beyond one or two waves of tiles."""
     x, y = xy
-    text = _check([x, y], C2C, direction, 21, seed=x)
-    columns = [l for l in text.splitlines() if "[1->1]" in l]
-    assert len(columns) == 1
-    few = x <= 32 and y <= (16 if x >= 9 else 32)
-    assert ("[pair tiles]" in columns[0]) == (not few), text
-    _check([x, 2 * y], R2C, direction, 21, seed=x)
-    _check([x, 2 * y], C2R, direction, 21, seed=x)
+    for batch in (21, 1300):
+        text = _check([x, y], C2C, direction, batch, seed=x)
+        columns = [l for l in text.splitlines() if "[1->1]" in l]
+        assert len(columns) == 1
+        few = x <= 32 and y <= (16 if x >= 9 else 32) and batch > 21
+        assert ("[pair tiles]" in columns[0]) == (not few), text
+    _check([x, 2 * y], R2C, direction, 1300, seed=x)
+    _check([x, 2 * y], C2R, direction, 1300, seed=x)
 
 
 @pytest.mark.parametrize("n", [17, 23, 31, 34, 37])
 @pytest.mark.parametrize("direction", [FWD, INV])
 def test_short_bluestein(cuda, n, direction):
-    """Convolutions of up to 64 points in two launches, longer ones in one kernel."""
+    """Convolutions of up to 64 points of more than 16 rows in two launches, others in one kernel."""
     for typ in (C2C, R2C, C2R):
-        text = _check([n], typ, direction, 333, seed=n)
-        assert ("in one kernel" in text) == (2 * n - 1 > 64), text
+        for batch in (3, 333):
+            text = _check([n], typ, direction, batch, seed=n)
+            assert ("in one kernel" in text) == (2 * n - 1 > 64 or batch == 3), text
 
 
 @pytest.mark.parametrize("n,batch,passes", [(4374, 8, 2), (4374, 900, 1), (4410, 8, 2), (4410, 900, 1), (4368, 900, 2),
