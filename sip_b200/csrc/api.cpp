@@ -690,7 +690,8 @@ int32_t asdFftPlanLaunchCount(void *handle)
     std::lock_guard<std::mutex> lock(p->mu);
     int32_t n = 0;
     for (const auto &s : p->steps) {
-        if (s.kind == sipfft::StepKind::kTile || s.kind == sipfft::StepKind::kTranspose)
+        if (s.kind == sipfft::StepKind::kTile || s.kind == sipfft::StepKind::kTranspose ||
+            s.kind == sipfft::StepKind::kBlueFused)
             n += 1;
         else
             n += static_cast<int32_t>((s.rows + 65534) / 65535);

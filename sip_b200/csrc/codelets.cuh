@@ -371,7 +371,7 @@ constexpr int crt_unit(int a, int b)
 // twiddles in between.  The pair tiles take larger radices than the one-transform tiles, and
 // the twiddles' 2 to 8 products would round more often (relative rms error of a radix, with
 // them -> without: 6 4.5e-8 -> 3.9e-8, 10 5.7e-8 -> 5.1e-8, 12 5.2e-8 -> 4.8e-8,
-// 14 6.0e-8 -> 5.5e-8, 15 6.3e-8 -> 5.7e-8; 1000-point rows 1.22e-7 -> 1.14e-7).
+// 14 6.0e-8 -> 5.5e-8, 15 6.3e-8 -> 5.7e-8; 1000-point rows 1.22e-7 -> 1.10e-7).
 // Else Cooley-Tukey, decimation in time: interleaved sub-sequences, twiddles W_R^(n1*k2),
 // output index k = k2 + B*k1.  (The one-transform kernels, which hold every radix at a
 // fixed register bound, lose 3 to 8 % with the other order: r2c 9216 x 455 36.6 -> 38.2 us.)

@@ -215,3 +215,10 @@ def test_tuned_sequence_without_a_pair_tile(cuda, tmp_path):
             f.write(json.dumps({"gpu": torch.cuda.get_device_name(0), "type": "c2c", "precision": "fp32", "n": n,
                                 "radices": [], "maxe": 0, "row_threads": 0, "us": 0, "plan_us": 0}) + "\n")
     assert fft.tune_cache_load(path) == len(entries)
+
+
+def test_launch_count_of_many_bluestein_rows(cuda):
+    """The one-kernel form is one launch whatever the number of rows."""
+    plan = fft.FftPlan([37], C2C, FWD, 70000)
+    assert "in one kernel" in plan.describe() and plan.launches() == 1
+    plan.close()
