@@ -462,7 +462,7 @@ struct Builder {
         if (!add_pair_variant(s, tuned ? &tc : nullptr)) return false;
         // against the step before it; the columns of a 2D C2R plan, whose rows end the
         // plan in ascending order, start at the end
-        if (s.cp_fn || (s.pair && !s.row_fn))
+        if (s.cp_fn || (s.pair && !s.pair_unaligned))
             s.descending = p.steps.empty() ? p.fft_type == 0x11 && p.sizes.size() == 2 : !p.steps.back().descending;
         // passes of a multi-pass transform keep the FP32 kernels: their tiles would run on the
         // single-tile tensor-core kernel, several times slower than the double-buffered FP32 passes
@@ -534,7 +534,9 @@ struct Builder {
             // r2c 8 20 -> 15, 10 16 -> 15, but 14 12 <- 15 and 22 10 <- 16).  Few rows leave the SMs
             // idle either way, and the pair tile's chain is shorter (8 points, device time: 5000
             // rows 2.8 <- 3.4, 30000 4.3 -> 3.8; 13 points 2.9 <- 4.1, 4.7 <- 4.8).
-            if (d.n < (d.io == IO_R2C_PACKED ? 6 : 14) && d.n_cols > 16384 && !p.use_tuned) return true;
+            // A source that the row kernel's bulk copies cannot read stays on pair tiles (4 M points
+            // at 8 bytes from alignment: c2c 3 points 34 us, 61).
+            s.pair_unaligned = d.n < (d.io == IO_R2C_PACKED ? 6 : 14) && d.n_cols > 16384 && !p.use_tuned;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
         } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32) &&
@@ -1560,7 +1562,7 @@ std::string describe_plan(const Plan &p)
     for (const Step &s : p.steps) {
         o << "  [" << static_cast<int>(s.src) << "->" << static_cast<int>(s.dst) << "] " << s.what;
         if (s.kind == StepKind::kTile) {
-            if (s.pair && !s.cp_fn && !s.row_fn && s.tc_fmt < 0) {
+            if (s.pair && !s.pair_unaligned && s.tc_fmt < 0) {
                 o << " [pair tiles] n=" << s.pd.n << " radices=";
                 for (int i = 0; i < s.pd.nstages; i++) o << (i ? "x" : "") << s.pd.st[i].R;
                 o << " pairs=" << s.pd.P << " tiles=" << s.pd.tiles << " grid=" << s.pair_grid

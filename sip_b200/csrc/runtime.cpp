@@ -322,6 +322,7 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
     for (const Step &s : steps) {
         const void *src = bufs[static_cast<int>(s.src)];
         void *dst = bufs[static_cast<int>(s.dst)];
+        const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
         if (src == nullptr || dst == nullptr) return cudaErrorInvalidDevicePointer;
         cudaError_t e = cudaSuccess;
         switch (s.kind) {
@@ -336,13 +337,13 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                     d.out = dst;
                     e = launch_tc(d, d.n, s.tc_fmt, s.forward, s.tc_mat, s.tc_tw, s.grid, device_error_word(p.device),
                                   st);
-                } else if (s.pair && !s.cp_fn && !s.row_fn && (!s.pd.rows || src != dst)) {
+                } else if (s.pair && (!s.pair_unaligned || !aligned) && (!s.pd.rows || src != dst)) {
                     PairDesc d = s.pd;
                     d.in = src;
                     d.out = dst;
                     d.descending = s.descending ? 1 : 0;
                     e = launch_pair(d, s.forward, s.pair_grid, st);
-                } else if (s.has_row && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && src != dst) {
+                } else if (s.has_row && aligned && src != dst) {
                     TileDesc d = s.rd;
                     d.in = src;
                     d.out = dst;
@@ -351,18 +352,11 @@ cudaError_t execute_steps(const Plan &p, const std::vector<Step> &steps, const v
                                              st);
                     else
                         e = launch_row_tiles(d, s.maxe, s.forward, s.row_grid, device_error_word(p.device), st);
-                } else if (s.cp_fn && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+                } else if (s.cp_fn && aligned) {
                     TileDesc d = s.cd;
                     d.in = src;
                     d.out = dst;
                     e = launch_col_pipe(s.cp_fn, d, s.cp_smem, s.cp_grid, s.descending, device_error_word(p.device), st);
-                } else if (s.pair && (!s.pd.rows || src != dst)) {
-                    // a source that the static engines' bulk copies cannot read
-                    PairDesc d = s.pd;
-                    d.in = src;
-                    d.out = dst;
-                    d.descending = s.descending ? 1 : 0;
-                    e = launch_pair(d, s.forward, s.pair_grid, st);
                 } else if (s.db) {
                     TileDesc d = s.d;
                     d.in = src;

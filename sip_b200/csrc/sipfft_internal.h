@@ -222,8 +222,9 @@ struct Step {
     // column and pair kernels: last tile first (each step walks against the one
     // before it, whose last outputs are still in L2)
     bool descending = false;
-    // runtime-radix pair tiles (no alignment requirement)
-    bool pair = false;
+    // runtime-radix pair tiles (no alignment requirement); pair_unaligned: only for a source
+    // that the step's other kernel cannot copy in bulk (8-byte aligned)
+    bool pair = false, pair_unaligned = false;
     PairDesc pd{};
     int pair_grid = 1;
     bool has_row = false;
