@@ -14,6 +14,10 @@ constexpr int kPairStages = 8;      // most stages of a tile
 constexpr int kPairMaxRadix = 16;   // radices 2..16
 constexpr int kPairBufBytes = 37504;  // most shared memory of one tile buffer (two per CTA, three CTAs per SM)
 constexpr int kPairBufBytes4 = 27264;  // the same for four CTAs per SM
+// Most columns (rows) of a step: a tile of 2 x 128 past the last column still has
+// indices below 2^31, as FastDiv needs them (the last tile's threads look the pass
+// twiddles of columns up that do not exist).
+constexpr int64_t kPairMaxCols = (int64_t(1) << 31) - 2 * kPairThreads;
 
 // Butterflies of radix R that a thread holds between a stage's gather and its
 // scatter: at most 16 points of two transforms (64 registers).

@@ -516,7 +516,7 @@ struct Builder {
         const TileDesc &d = s.d;
         const bool rows = !d.xfast;
         const int64_t most = int64_t(1) << 31;
-        if (d.n < 2 || d.n_cols >= most || d.n_outer >= most) return true;
+        if (d.n < 2 || d.n_cols > kPairMaxCols || d.n_outer >= most) return true;
         // Columns with a compile-time engine keep it: the TMA tiles, and for strides those
         // cannot read (odd ones, as the half spectra of R2C plans have) the element-copy
         // tiles (r2c 512^2 x 16 28 us, 32 on pair tiles; 128^2 x 256 29, 30)
@@ -1000,7 +1000,7 @@ struct Builder {
         // launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317; c2c 17 x 1 4.6 / 18,
         // c2r 17 x 64 25 / 21).
         PairChoice fused;
-        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= 16) && rows < (int64_t(1) << 31)) {
+        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= 16) && rows <= kPairMaxCols) {
             const int64_t pow2 = m;
             double best = 1e30;
             for (int64_t f : {1, 3, 5, 7, 9, 15}) {

@@ -232,6 +232,18 @@ int main()
                 ok = false;
             }
         }
+    // ... up to the last index of a tile that starts at the largest column, by powers of two (the
+    // divisors whose reciprocal has the largest error) and their neighbours
+    for (int64_t v = 1; v < int64_t(1) << 31; v *= 2)
+        for (int64_t w : {v, v - 1, v + 1})
+            for (int64_t m = kPairMaxCols - 64; m < kPairMaxCols + 2 * kPairThreads; m++) {
+                if (w < 1) continue;
+                const FastDiv f = fast_div(w);
+                if (f.div(static_cast<uint32_t>(m)) != m / w) {
+                    std::printf("FAILED division %lld / %lld\n", (long long)m, (long long)w);
+                    ok = false;
+                }
+            }
     std::printf("%d shapes %s\n", shapes, ok ? "ALL OK" : "FAILED");
     return ok ? 0 : 1;
 }
