@@ -160,8 +160,9 @@ bool save_tune_cache(const std::string &path, int device)
     return static_cast<bool>(o);
 }
 
-// Candidate radix orders / elements per thread for one length.
-std::vector<TuneChoice> tune_candidates(int64_t n)
+// Candidate radix orders / elements per thread for one length; on the pair kernel, which
+// takes the radices and a tile size only, radix orders and two tile sizes.
+std::vector<TuneChoice> tune_candidates(int64_t n, bool pairs)
 {
     std::vector<TuneChoice> out;
     std::vector<int> base;
@@ -203,7 +204,7 @@ std::vector<TuneChoice> tune_candidates(int64_t n)
     for (const auto &o : orders) {
         for (int maxe : {8, 16}) {
             const int tpt = static_cast<int>((n + maxe - 1) / maxe);
-            if (tpt > kBatchBlock) continue;
+            if (tpt > kBatchBlock || (pairs && maxe != 16)) continue;
             // tile shape: transforms per tile so that a tile has about this many threads
             // (the batch kernel's CTA has 256)
             for (int threads : {128, 256}) {
@@ -225,6 +226,7 @@ struct BatchPlan {
     bool forward = true;
     std::vector<int64_t> sizes, batches;
     std::vector<BatchSeg> segs;
+    bool allow_pairs = true;  // (the autotuner times lengths on the kernel that the whole set runs on)
     bool pairs = false;  // every segment is a pair tile (two transforms per thread): pair_segs instead of segs
     std::vector<PairSeg> pair_segs;
     std::vector<int2> items;
@@ -405,10 +407,13 @@ std::string build_batch_with(BatchPlan &bp)
     }
     *bp.status = 0;
     if (const char *s = std::getenv("ASDSIP_FFT_BATCH_POLLS")) bp.polls = static_cast<uint32_t>(std::atoll(s));
-    size_t bytes = bp.segs.size() * sizeof(BatchSeg);
-    if (cudaMalloc(&bp.d_segs, bytes) != cudaSuccess ||
-        cudaMemcpy(bp.d_segs, bp.segs.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMalloc(&bp.d_items, bp.items.size() * sizeof(int2)) != cudaSuccess ||
+    const size_t bytes = bp.segs.size() * sizeof(BatchSeg);
+    if (!bp.pairs && (cudaMalloc(&bp.d_segs, bytes) != cudaSuccess ||
+                      cudaMemcpy(bp.d_segs, bp.segs.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess)) {
+        cudaGetLastError();
+        return "twiddle table: device allocation failed";
+    }
+    if (cudaMalloc(&bp.d_items, bp.items.size() * sizeof(int2)) != cudaSuccess ||
         cudaMemcpy(bp.d_items, bp.items.data(), bp.items.size() * sizeof(int2), cudaMemcpyHostToDevice) !=
             cudaSuccess ||
         cudaMalloc(&bp.d_counters, (kBatchDone + bp.segs.size()) * sizeof(int)) != cudaSuccess) {
@@ -426,7 +431,8 @@ std::string build_batch_with(BatchPlan &bp)
 std::string build_batch(BatchPlan &bp)
 {
     std::vector<int> probe;
-    bp.pairs = std::all_of(bp.sizes.begin(), bp.sizes.end(), [&](int64_t n) { return n > 1 && factor_radices(n, probe); });
+    bp.pairs = bp.allow_pairs && std::all_of(bp.sizes.begin(), bp.sizes.end(),
+                                             [&](int64_t n) { return n > 1 && factor_radices(n, probe); });
     if (bp.pairs) {
         std::string e = build_batch_with(bp);
         if (e != kNoPairs) return e;
@@ -511,10 +517,11 @@ bool time_mix(const std::vector<int64_t> &sizes, const std::vector<int64_t> &row
 // launch every segment shares the grid and the CTA's shared memory is sized
 // by the largest tile of any segment, so a winner's tile shape and radix
 // order are kept only if the launch of all the groups together runs faster
-// with them (lengths taken by decreasing bytes; the arithmetic choice of
+// with them (lengths taken by decreasing weight; the arithmetic choice of
 // precision mode 3 is kept either way).
+// weight: points of the launch whose tiles each tuned length shapes.
 void accept_in_mix(const std::vector<int64_t> &sizes, const std::vector<int64_t> &rows_per,
-                   const std::vector<int64_t> &targets, bool forward, int device, cudaEvent_t e0, cudaEvent_t e1)
+                   const std::map<int64_t, int64_t> &weight, bool forward, int device, cudaEvent_t e0, cudaEvent_t e1)
 {
     int64_t total = 0;
     for (size_t i = 0; i < sizes.size(); i++) total += sizes[i] * rows_per[i];
@@ -526,20 +533,14 @@ void accept_in_mix(const std::vector<int64_t> &sizes, const std::vector<int64_t>
         return;  // no room for the whole mix: the per-length winners stand
     }
     cudaMemset(in, 0, total * sizeof(float2));
-    // bytes of the launch whose tiles each tuned length shapes (as a group or as a pass)
-    std::map<int64_t, int64_t> weight;
-    for (size_t i = 0; i < sizes.size(); i++) {
-        if (sizes[i] <= kBatchMaxRowN) weight[sizes[i]] += sizes[i] * rows_per[i];
-        else
-            for (int r : multipass_split(sizes[i])) weight[r] += sizes[i] * rows_per[i];
-    }
-    std::vector<std::pair<int64_t, int64_t>> order;  // (bytes, length)
+    std::vector<std::pair<int64_t, int64_t>> order;  // (weight, length)
     std::map<int64_t, TuneChoice> winners;
-    for (const int64_t n : targets) {
+    for (const auto &w : weight) {
+        const int64_t n = w.first;
         TuneChoice c;
         if (!tuned_choice(n, c) || c.radices.empty()) continue;
         winners[n] = c;
-        order.push_back({weight[n], n});
+        order.push_back({w.second, n});
         TuneChoice plain = c;  // the planner's defaults for the launch, the arithmetic kept
         plain.radices.clear();
         plain.maxe = 0;
@@ -593,33 +594,57 @@ int autotune_lengths(const std::vector<int64_t> &sizes, const std::vector<int64_
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    // The lengths whose tiles the uneven-batch kernel runs: groups of at most
-    // 16384 points, and the pass lengths of the multi-pass split of longer rows
-    // (their passes are column tiles of those lengths)
-    std::vector<int64_t> targets;
-    for (int64_t n : sizes) {
-        if (n <= 16384) targets.push_back(n);
-        if (n > kBatchMaxRowN)
-            for (int r : multipass_split(n)) targets.push_back(r);
+    // The lengths of the tiles that the set's launch runs (weight: their points): groups that
+    // are one tile, and the passes of longer rows.  Other groups of at most 16384 points have
+    // no tile of their own; of them only the arithmetic of the ordinary plan is chosen.
+    std::map<int64_t, int64_t> weight;
+    bool pairs = false;
+    {
+        BatchPlan set;
+        set.device = device;
+        set.forward = forward;
+        set.sizes = sizes;
+        set.batches = rows_per;
+        if (build_batch(set).empty()) {
+            pairs = set.pairs;
+            for (size_t i = 0; i < set.segs.size(); i++) {
+                const TileDesc &d = set.segs[i].d;
+                weight[d.n] += d.n * d.n_cols * d.n_outer;
+            }
+        }
+        cudaGetLastError();
     }
-    std::sort(targets.begin(), targets.end());
-    targets.erase(std::unique(targets.begin(), targets.end()), targets.end());
-    for (const int64_t n : targets) {
-        TuneChoice best;
+    std::vector<int64_t> lengths;
+    for (const auto &w : weight) lengths.push_back(w.first);
+    for (int64_t n : sizes)
+        if (n <= 16384 && weight.find(n) == weight.end()) lengths.push_back(n);
+    std::sort(lengths.begin(), lengths.end());
+    lengths.erase(std::unique(lengths.begin(), lengths.end()), lengths.end());
+    for (const int64_t n : lengths) {
+        TuneChoice best, before;
         best.us = 1e30;
+        const bool known = tuned_choice(n, before);
+        const bool tile = weight.find(n) != weight.end() && n <= (pairs ? kPairMaxRowN : kBatchMaxRowN);
         // enough transforms that a launch is not just its overhead
         const int64_t rows = std::max<int64_t>(16, std::min<int64_t>((int64_t(1) << 22) / n, 4096));
-        for (TuneChoice c : tune_candidates(n)) {
+        for (TuneChoice c : tile ? tune_candidates(n, pairs) : std::vector<TuneChoice>()) {
             set_tuned_choice(n, c);
             // the uneven-batch kernel runs these tiles: time a one-group batch plan
             BatchPlan bp;
             bp.device = device;
             bp.forward = forward;
+            bp.allow_pairs = pairs;
             bp.sizes = {n};
             bp.batches = {rows};
             if (!build_batch(bp).empty()) {
                 cudaGetLastError();
                 continue;
+            }
+            if (pairs) {  // an order without a pair tile ran the planner's own: not a candidate
+                const PairDesc &q = bp.pair_segs[0].d;
+                bool same = bp.pairs && q.nstages == static_cast<int>(c.radices.size());
+                for (int i = 0; same && i < q.nstages; i++) same = q.st[i].R == c.radices[i];
+                if (!same) continue;
             }
             void *ws = nullptr;
             if (bp.ws_bytes && cudaMalloc(&ws, bp.ws_bytes) != cudaSuccess) {
@@ -642,10 +667,16 @@ int autotune_lengths(const std::vector<int64_t> &sizes, const std::vector<int64_
             c.us = ms * 1e3 / 5.0;
             if (c.us < best.us) best = c;
         }
+        if (tile && best.us >= 1e29) set_tuned_choice(n, known ? before : TuneChoice());
         // whole-plan arithmetic per length (ordinary plans in precision mode 3):
         // the FP32 kernels against the split-precision tensor-core forms
         TcConfig tcc;
-        if (best.us < 1e29 && (tc_config(static_cast<int>(n), tcc) || tc_rows_config(static_cast<int>(n), tcc))) {
+        if (tc_config(static_cast<int>(n), tcc) || tc_rows_config(static_cast<int>(n), tcc)) {
+            if (best.us >= 1e29) {
+                best = TuneChoice();
+                best.us = 0.0;
+                best.maxe = best.row_threads = 0;
+            }
             best.plan_us = 1e30;
             for (int form = 0; form < 3; form++) {
                 Plan q;
@@ -682,7 +713,7 @@ int autotune_lengths(const std::vector<int64_t> &sizes, const std::vector<int64_
     }
     cudaFree(buf);
     cudaFree(out);
-    accept_in_mix(sizes, rows_per, targets, forward, device, e0, e1);
+    accept_in_mix(sizes, rows_per, weight, forward, device, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return tuned;
@@ -870,13 +901,18 @@ int32_t asdFftAutotune(const int64_t *sizes, const int64_t *rows, int32_t n, int
         cudaGetLastError();
         return AsdSip::ACL_ERROR_INTERNAL_ERROR;
     }
-    std::vector<int64_t> s(sizes, sizes + n), r(rows, rows + n);
-    for (auto &x : r) x = std::max<int64_t>(1, std::min<int64_t>(x, 256));
-    std::string err;
-    sipfft::autotune_lengths(s, r, direction == AsdSip::ASCEND_FFT_FORWARD, dev, &err);
-    if (!err.empty()) return AsdSip::ACL_ERROR_INTERNAL_ERROR;
-    if (cache_path && *cache_path && !sipfft::save_tune_cache(cache_path, dev)) return AsdSip::ACL_ERROR_INTERNAL_ERROR;
-    return AsdSip::ACL_SUCCESS;
+    try {
+        std::vector<int64_t> s(sizes, sizes + n), r(rows, rows + n);
+        for (auto &x : r) x = std::max<int64_t>(1, std::min<int64_t>(x, 256));
+        std::string err;
+        sipfft::autotune_lengths(s, r, direction == AsdSip::ASCEND_FFT_FORWARD, dev, &err);
+        if (!err.empty()) return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+        if (cache_path && *cache_path && !sipfft::save_tune_cache(cache_path, dev))
+            return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+        return AsdSip::ACL_SUCCESS;
+    } catch (...) {
+        return AsdSip::ACL_ERROR_INTERNAL_ERROR;
+    }
 }
 
 int32_t asdFftTuneCacheLoad(const char *cache_path)

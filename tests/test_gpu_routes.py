@@ -227,3 +227,34 @@ def test_launch_count_of_many_bluestein_rows(cuda):
     plan = fft.FftPlan([37], C2C, FWD, 70000)
     assert "in one kernel" in plan.describe() and plan.launches() == 1
     plan.close()
+
+
+def test_autotune_takes_the_lengths_that_have_tiles(cuda, tmp_path):
+    """The tuner's lengths are those of the launch's tiles: passes as the planner splits them,
+    and no rows that are two passes."""
+    import json
+    import re
+
+    import torch
+
+    path = str(tmp_path / "tune.jsonl")
+    groups = [(2200, 40), (4400, 20), (1470, 64), (735, 64), (14300, 9)]
+    plan = fft.BatchPlan(groups, INV)
+    assert "kernel=pairs" in plan.describe()
+    tiles = {int(n) for n in re.findall(r" n=(\d+) tiles=", plan.describe())}
+    plan.close()
+    assert fft.autotune(groups, INV, path) == fft.ACL_SUCCESS
+    lines = [json.loads(l) for l in open(path)]
+    assert tiles <= {l["n"] for l in lines}
+    assert not {2200, 4400, 14300} & {l["n"] for l in lines}
+    plan = fft.BatchPlan(groups, INV, path)
+    assert "kernel=pairs" in plan.describe()
+    rng = np.random.default_rng(6)
+    x = (rng.uniform(-1, 1, plan.total) + 1j * rng.uniform(-1, 1, plan.total)).astype(np.complex64)
+    y = torch.zeros(plan.total, dtype=torch.complex64, device="cuda")
+    plan(torch.from_numpy(x).cuda(), y)
+    plan.synchronize()
+    for (n, b), off in zip(plan.groups, plan.offsets):
+        got = y[off:off + n * b].cpu().numpy().reshape(b, n)
+        assert oracle.rel_l2(got, oracle.c2c(x[off:off + n * b].reshape(b, n), False)) <= oracle.tolerance(n)
+    plan.close()
