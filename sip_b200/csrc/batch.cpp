@@ -387,7 +387,7 @@ std::string build_batch_with(BatchPlan &bp)
     if (bp.items.size() > 0x7fffffff) return "too many tiles";
     if (bp.pairs) {
         bp.block = kPairThreads;
-        bp.smem = pair_smem(bp.buf_words);
+        bp.smem = pair_smem_bytes(bp.buf_words);
     }
     const int per_sm = kernel_blocks_per_sm(bp.pairs ? pair_batch_fn(bp.forward) : batch_kernel_fn(bp.forward, bp.compact),
                                             bp.block, bp.smem);

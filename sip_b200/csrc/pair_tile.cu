@@ -24,7 +24,7 @@ void pair_kernel_fns(std::vector<const void *> &out)
     out.push_back(pair_blue_fn());
 }
 
-size_t pair_smem(int buf_words)
+size_t pair_smem_bytes(int buf_words)
 {
     const size_t head = ((kPairSlots * ((sizeof(PairSeg) + 15) / 16)) + 7) / 8 * 8;
     return (head + size_t(2) * buf_words) * 16;
@@ -32,7 +32,7 @@ size_t pair_smem(int buf_words)
 
 cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st)
 {
-    const size_t smem = pair_smem(d.buf_words);
+    const size_t smem = pair_smem_bytes(d.buf_words);
     if (grid <= 0 || d.tiles == 0 || smem > static_cast<size_t>(kMaxSmemBytes)) return cudaErrorInvalidConfiguration;
     PairSeg g{};
     g.d = d;
@@ -42,7 +42,7 @@ cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t 
 
 cudaError_t launch_pair_blue(const PairBlue &q, int grid, cudaStream_t st)
 {
-    const size_t smem = pair_smem(q.g.d.buf_words);
+    const size_t smem = pair_smem_bytes(q.g.d.buf_words);
     if (grid <= 0 || q.g.d.tiles == 0 || smem > static_cast<size_t>(kMaxSmemBytes)) return cudaErrorInvalidConfiguration;
     PairBlue g = q;
     void *args[] = {&g};
@@ -54,7 +54,7 @@ cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, cons
 {
     BatchBufs b = bufs;
     void *args[] = {&segs, &items, &nitems, &words, &b, &err, &buf_words, &polls};
-    return cudaLaunchKernel(pair_batch_fn(forward), dim3(grid), dim3(kPairThreads), args, pair_smem(buf_words), st);
+    return cudaLaunchKernel(pair_batch_fn(forward), dim3(grid), dim3(kPairThreads), args, pair_smem_bytes(buf_words), st);
 }
 
 }  // namespace sipfft

@@ -148,6 +148,32 @@ inline bool pair_shape(PairDesc &d, int n, const int *radix, int nstages, bool r
     return ns == n;
 }
 
+// Butterfly b of thread tid in a stage of `tasks` butterflies, nbf of each transform: pair p,
+// index j; off (and butterfly 0) beyond the tile.  E: the elements fastest, else the pairs.
+struct PairTask {
+    int p, j;
+    bool on;
+};
+template <bool E>
+__host__ __device__ __forceinline__ PairTask pair_task(int tid, int b, int lp, int nbf, uint32_t nbf_m, int tasks)
+{
+    if constexpr (E) {
+        const int i = tid + b * kPairThreads;
+        const bool on = i < tasks;
+        const int u = on ? i : 0;
+#ifdef __CUDA_ARCH__
+        const int p = nbf == 1 ? u : static_cast<int>(__umulhi(static_cast<uint32_t>(u), nbf_m));
+#else
+        const int p = nbf == 1 ? u : static_cast<int>((uint64_t(uint32_t(u)) * nbf_m) >> 32);
+#endif
+        return {p, u - p * nbf, on};
+    } else {
+        const int j = (tid >> lp) + b * (kPairThreads >> lp);
+        const bool on = j < nbf;
+        return {tid & ((1 << lp) - 1), on ? j : 0, on};
+    }
+}
+
 // Work-tile words of butterfly (p, j) of stage t: its first input (the others
 // follow t.gstep apart) and its first output (ns * SE apart).
 __host__ __device__ __forceinline__ int pair_gather_at(int SP, int SE, int gpad, int p, int j, int q)

@@ -138,23 +138,12 @@ __device__ __noinline__ void pair_stage(int stage, bool to_global, const PairTil
     const int nbf = t.nbf, ns = FIRST ? 1 : t.ns, lp = d.lp, tasks = t.tasks, SP = d.SP, SE = d.SE, spad = t.spad;
     const uint32_t ns_m = t.ns_m, nbf_m = t.nbf_m;
     cpx2 v[NB * R];
-    // butterfly b of this thread: pair p, index j; false beyond the tile
-    const int p0 = tid & ((1 << lp) - 1), j0 = tid >> lp, dj = kPairThreads >> lp;
+    const int p0 = tid & ((1 << lp) - 1);
     auto task = [&](int b, int &p, int &j) -> bool {
-        if constexpr (E) {
-            const int i = tid + b * kPairThreads;
-            const bool on = i < tasks;
-            const int u = on ? i : 0;
-            p = nbf == 1 ? u : static_cast<int>(__umulhi(static_cast<uint32_t>(u), nbf_m));
-            j = u - p * nbf;
-            return on;
-        } else {
-            p = p0;
-            j = j0 + b * dj;
-            const bool on = j < nbf;
-            j = on ? j : 0;
-            return on;
-        }
+        const PairTask k = pair_task<E>(tid, b, lp, nbf, nbf_m, tasks);
+        p = k.p;
+        j = k.j;
+        return k.on;
     };
     auto block = [&](int j) { return FIRST ? j : static_cast<int>(__umulhi(static_cast<uint32_t>(j), ns_m)); };  // j div ns
     PassTwiddle tw{};

@@ -582,7 +582,7 @@ struct Builder {
         if (!ok) return true;
         const int64_t per_outer = (d.n_cols + 2 * q.P - 1) / (2 * q.P), tiles = per_outer * d.n_outer;
         if (tiles >= most) return true;
-        const int per_sm = kernel_blocks_per_sm(pair_kernel_fn(s.forward), kPairThreads, pair_smem(q.buf_words));
+        const int per_sm = kernel_blocks_per_sm(pair_kernel_fn(s.forward), kPairThreads, pair_smem_bytes(q.buf_words));
         if (per_sm <= 0) return true;
         q.io = d.io;
         q.n_cols = d.n_cols;
@@ -1104,7 +1104,7 @@ struct Builder {
         if (!t) return false;
         p.tables.push_back(t);
         q.stw = t->ptr;
-        const int per_sm = std::max(1, kernel_blocks_per_sm(pair_blue_fn(), kPairThreads, pair_smem(q.buf_words)));
+        const int per_sm = std::max(1, kernel_blocks_per_sm(pair_blue_fn(), kPairThreads, pair_smem_bytes(q.buf_words)));
         s.pair_grid = per_sm * sm_count(device);
         std::ostringstream w;
         w << "Bluestein n=" << n << " via M=" << m << " rows=" << rows << " in one kernel, radices=";
@@ -1556,7 +1556,7 @@ std::string describe_plan(const Plan &p)
                 o << " [pair tiles] n=" << s.pd.n << " radices=";
                 for (int i = 0; i < s.pd.nstages; i++) o << (i ? "x" : "") << s.pd.st[i].R;
                 o << " pairs=" << s.pd.P << " tiles=" << s.pd.tiles << " grid=" << s.pair_grid
-                  << " smem=" << pair_smem(s.pd.buf_words) << "\n";
+                  << " smem=" << pair_smem_bytes(s.pd.buf_words) << "\n";
                 continue;
             }
             o << (s.cp_fn ? " [TMA column tiles, static engine]"

@@ -95,7 +95,7 @@ const void *pair_batch_fn(bool forward);
 const void *pair_blue_fn();
 cudaError_t launch_pair_blue(const PairBlue &q, int grid, cudaStream_t st);
 void pair_kernel_fns(std::vector<const void *> &out);
-size_t pair_smem(int buf_words);
+size_t pair_smem_bytes(int buf_words);
 cudaError_t launch_pair(const PairDesc &d, bool forward, int grid, cudaStream_t st);
 cudaError_t launch_pair_batch(int grid, int buf_words, const PairSeg *segs, const int2 *items, int nitems,
                               int *words, const BatchBufs &bufs, int *err, uint32_t polls, bool forward,

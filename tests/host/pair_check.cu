@@ -59,19 +59,10 @@ static bool run(int n, const std::vector<int> &rad, bool rows, bool runs, int64_
         for (int phase = 0; phase < 2; phase++)
             for (int tid = 0; tid < kPairThreads; tid++)
                 for (int b = 0; b < nb; b++) {
-                    int i = tid + b * kPairThreads;
-                    bool on = i < t.tasks;
-                    if (!on) i = 0;
-                    int p, j;
-                    if (!fast_e) {
-                        p = tid & (d.P - 1);
-                        j = (tid >> d.lp) + b * (kPairThreads >> d.lp);
-                        CHECK((j < t.nbf) == on);
-                        if (!on) j = 0;
-                    } else {
-                        p = t.nbf == 1 ? i : static_cast<int>((uint64_t(uint32_t(i)) * t.nbf_m) >> 32);
-                        j = i - p * t.nbf;
-                    }
+                    const PairTask k0 = fast_e ? pair_task<true>(tid, b, d.lp, t.nbf, t.nbf_m, t.tasks)
+                                               : pair_task<false>(tid, b, d.lp, t.nbf, t.nbf_m, t.tasks);
+                    const int p = k0.p, j = k0.j;
+                    const bool on = k0.on;
                     const int q = s == 0 ? j : static_cast<int>((uint64_t(uint32_t(j)) * t.ns_m) >> 32);
                     CHECK(p >= 0 && p < d.P && j >= 0 && j < t.nbf && q == j / t.ns);
                     cd *a = &v[(size_t(tid) * nb + b) * t.R];
