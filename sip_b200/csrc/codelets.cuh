@@ -13,7 +13,7 @@
 // multiply and FMA do two transforms' arithmetic in one issue slot at the
 // FP32 pipe's full rate (measured: 16 FFMA and 8 packed FMA take the same
 // pipe time in half the slots).  Both run the same operations in the same
-// order, so their results agree bit for bit, but for the composite radices (Comp).
+// order, so their results agree bit for bit, but for the composite radices (CompPrime).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -365,36 +365,23 @@ constexpr int crt_unit(int a, int b)
     return x;
 }
 
-// Composite radix R = A*B in registers: B-point DFTs, then A-point DFTs.
-// Two transforms at once, coprime A and B (every composite radix of the kernels): the
-// prime-factor form, whose input B n1 + A n2 and output k = k1 (mod A) = k2 (mod B) need no
-// twiddles in between.  The pair tiles take larger radices than the one-transform tiles, and
-// the twiddles' 2 to 8 products would round more often (relative rms error of a radix, with
-// them -> without: 6 4.5e-8 -> 3.9e-8, 10 5.7e-8 -> 5.1e-8, 12 5.2e-8 -> 4.8e-8,
-// 14 6.0e-8 -> 5.5e-8, 15 6.3e-8 -> 5.7e-8; 1000-point rows 1.22e-7 -> 1.10e-7).
-// Else Cooley-Tukey, decimation in time: interleaved sub-sequences, twiddles W_R^(n1*k2),
-// output index k = k2 + B*k1.  (The one-transform kernels, which hold every radix at a
-// fixed register bound, lose 3 to 8 % with the other order: r2c 9216 x 455 36.6 -> 38.2 us.)
-template <int A, int B, bool FWD, class V>
+// Composite radix R = A*B in registers (Cooley-Tukey, decimation in time):
+// B-point DFTs over the A interleaved sub-sequences, twiddles W_R^(n1*k2),
+// then A-point DFTs; output index k = k2 + B*k1.
+template <int A, int B, bool FWD>
 struct Comp {
     static constexpr int R = A * B;
-    static constexpr bool kCoprime = common_divisor(A, B) == 1 && sizeof(V) == sizeof(cpx2);
-    SIPFFT_HD static constexpr int input(int n1, int n2) { return kCoprime ? (B * n1 + A * n2) % R : n1 + A * n2; }
-    SIPFFT_HD static constexpr int output(int k1, int k2)
-    {
-        if constexpr (kCoprime) return (k1 * crt_unit(A, B) + k2 * crt_unit(B, A)) % R;
-        return k2 + B * k1;
-    }
+    template <class V>
     SIPFFT_HD static void run(V *a)
     {
         V y[A][B];
 #pragma unroll
         for (int n1 = 0; n1 < A; n1++) {
 #pragma unroll
-            for (int n2 = 0; n2 < B; n2++) y[n1][n2] = a[input(n1, n2)];
+            for (int n2 = 0; n2 < B; n2++) y[n1][n2] = a[n1 + A * n2];
             dft<B, FWD>(y[n1]);
         }
-        if constexpr (!kCoprime) twiddle<1, 1>(y);
+        twiddle<1, 1>(y);
 #pragma unroll
         for (int k2 = 0; k2 < B; k2++) {
             V z[A];
@@ -402,10 +389,10 @@ struct Comp {
             for (int n1 = 0; n1 < A; n1++) z[n1] = y[n1][k2];
             dft<A, FWD>(z);
 #pragma unroll
-            for (int k1 = 0; k1 < A; k1++) a[output(k1, k2)] = z[k1];
+            for (int k1 = 0; k1 < A; k1++) a[k2 + B * k1] = z[k1];
         }
     }
-    template <int N1, int K2>
+    template <int N1, int K2, class V>
     SIPFFT_HD static void twiddle(V (&y)[A][B])
     {
         if constexpr (N1 < A) {
@@ -419,13 +406,49 @@ struct Comp {
     }
 };
 
+// The same of coprime A and B (every composite radix of the kernels) on two transforms, in the
+// prime-factor order: input B n1 + A n2 and output k = k1 (mod A) = k2 (mod B) need no twiddles.
+// The pair tiles take larger radices than the one-transform tiles, and the twiddles' 2 to 8
+// products would round more often (relative rms error of a radix, with them -> without:
+// 6 4.5e-8 -> 3.9e-8, 10 5.7e-8 -> 5.1e-8, 12 5.2e-8 -> 4.8e-8, 14 6.0e-8 -> 5.5e-8,
+// 15 6.3e-8 -> 5.7e-8; 1000-point rows 1.22e-7 -> 1.10e-7).  (The one-transform kernels, which
+// hold every radix at a fixed register bound, lose 3 to 8 % in this order: r2c 9216 x 455
+// 36.6 -> 38.2 us.)
+template <int A, int B, bool FWD>
+struct CompPrime {
+    static constexpr int R = A * B, K1 = crt_unit(A, B), K2 = crt_unit(B, A);
+    SIPFFT_HD static void run(cpx2 *a)
+    {
+        cpx2 y[A][B];
+#pragma unroll
+        for (int n1 = 0; n1 < A; n1++) {
+#pragma unroll
+            for (int n2 = 0; n2 < B; n2++) y[n1][n2] = a[(B * n1 + A * n2) % R];
+            dft<B, FWD>(y[n1]);
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) {
+            cpx2 z[A];
+#pragma unroll
+            for (int n1 = 0; n1 < A; n1++) z[n1] = y[n1][k2];
+            dft<A, FWD>(z);
+#pragma unroll
+            for (int k1 = 0; k1 < A; k1++) a[(k1 * K1 + k2 * K2) % R] = z[k1];
+        }
+    }
+};
+
 template <int R, bool FWD, class V>
 SIPFFT_HD void dft(V *a)
 {
     if constexpr (is_pow2<R>()) {
         Pow2<R, FWD>::run(a);
     } else if constexpr (R % 2 == 0 || (smallest_prime_factor(R) != R && R > 13)) {
-        Comp<comp_first(R), R / comp_first(R), FWD, V>::run(a);
+        constexpr int A = comp_first(R), B = R / A;
+        if constexpr (sizeof(V) == sizeof(cpx2) && common_divisor(A, B) == 1)
+            CompPrime<A, B, FWD>::run(a);
+        else
+            Comp<A, B, FWD>::run(a);
     } else {
         Odd<R, FWD>::run(a);
     }
