@@ -101,7 +101,7 @@ AspbStatus finish_plan(sipfft::Plan &p, std::string (*builder)(sipfft::Plan &), 
     p.c32_steps.clear();
     p.c32_base.clear();
     p.c32_state = 0;
-    p.pair_route = false;
+    p.pair_route = p.tile_first = false;
     for (size_t &b : p.ws_buf_bytes) b = 0;
     if (builder != sipfft::build_plan_istft) p.istft = false;
     p.ws_bytes = 0;
@@ -210,9 +210,10 @@ AspbStatus run(sipfft::Plan &p, const void *in, void *out, const char *where, co
     int cur = 0;
     cudaGetDevice(&cur);
     if (cur != p.device) cudaSetDevice(p.device);
-    cudaError_t e = complex32 ? sipfft::execute_steps(p, p.c32_steps, in, out, p.workspace,
-                                                      static_cast<cudaStream_t>(p.stream))
-                              : sipfft::execute_plan(p, in, out, static_cast<cudaStream_t>(p.stream), in_im, out_im);
+    const bool tile = p.tile_first && in != out && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+    cudaError_t e = complex32 || tile ? sipfft::execute_steps(p, complex32 ? p.c32_steps : p.c32_base, in, out,
+                                                              p.workspace, static_cast<cudaStream_t>(p.stream))
+                                      : sipfft::execute_plan(p, in, out, static_cast<cudaStream_t>(p.stream), in_im, out_im);
     if (cur != p.device) cudaSetDevice(cur);
     if (e != cudaSuccess) {
         log_error(where, cudaGetErrorString(e));
@@ -689,7 +690,7 @@ int32_t asdFftPlanLaunchCount(void *handle)
     if (!p) return -1;
     std::lock_guard<std::mutex> lock(p->mu);
     int32_t n = 0;
-    for (const auto &s : p->steps) {
+    for (const auto &s : p->tile_first ? p->c32_base : p->steps) {
         if (s.kind == sipfft::StepKind::kTile || s.kind == sipfft::StepKind::kTranspose ||
             s.kind == sipfft::StepKind::kBlueFused)
             n += 1;

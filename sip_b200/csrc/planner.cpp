@@ -531,12 +531,13 @@ struct Builder {
             // Many rows of a few points: a tile's fixed work is spread over too little, and the
             // one-transform tile kernel is faster (4 M points, us, pair tiles -> tile kernel: c2c
             // 2 points 51 -> 31, 5 28 -> 23, 12 31 -> 26, 13 26 -> 25, 14 27 <- 31; c2r 22 20 -> 18;
-            // r2c 8 20 -> 15, 10 16 -> 15, but 14 12 <- 15 and 22 10 <- 16).  Few rows leave the SMs
+            // r2c 8 20 -> 15, 10 16 -> 15, 16 20 -> 17, but 14 12 <- 15 and 22 10 <- 16).  Few rows leave the SMs
             // idle either way, and the pair tile's chain is shorter (8 points, device time: 5000
             // rows 2.8 <- 3.4, 30000 4.3 -> 3.8; 13 points 2.9 <- 4.1, 4.7 <- 4.8).
             // A source that the row kernel's bulk copies cannot read stays on pair tiles (4 M points
             // at 8 bytes from alignment: c2c 3 points 34 us, 61).
-            s.pair_unaligned = d.n < (d.io == IO_R2C_PACKED ? 6 : 14) && d.n_cols > 16384 && !p.use_tuned;
+            const bool few = d.io == IO_R2C_PACKED ? d.n < 6 || d.n == 8 : d.n < 14;
+            s.pair_unaligned = few && d.n_cols > 16384 && !p.use_tuned;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
         } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32) &&
@@ -660,13 +661,17 @@ struct Builder {
     //   have an odd distance (4410 45 -> 49);
     // * beyond L2 the second pass's traffic shows: only multiples of 16, whose passes keep
     //   16-byte copies and whole sectors (4410 297 -> 338, 6084 274 -> 331; 4368 322 -> 282).
-    bool long_row_in_two(int64_t n, int64_t outer) const
+    // In place and from an unaligned source the one tile runs unpipelined, and two passes are faster
+    // throughout (4410 x 951 in place 74 -> 47): 1D plans hold both.
+    // `fits`: the length splits and its workspace fits.
+    bool long_row_in_two(int64_t n, int64_t outer, bool &fits) const
     {
         std::vector<int> one, two;
         double cost;
-        if (n % 2 || !factor_radices(n, one) || !pair_split(n, kPairBufBytes, two, cost)) return false;
         const int64_t bytes = copies_bytes(n, outer);
-        if (bytes / 3 > spare_copy_bytes(device)) return false;  // (no workspace)
+        fits = n % 2 == 0 && factor_radices(n, one) && bytes / 3 <= spare_copy_bytes(device) &&
+               pair_split(n, kPairBufBytes, two, cost);
+        if (!fits) return false;
         if (n >= 6800 || one.size() >= 5 || bytes <= kL2Bytes / 2) return true;
         if (bytes <= kL2Bytes) return cost <= 205 && (two[1] % 2 == 0 || n % 8 == 0 || n >= 4500);
         return cost <= 190 && n % 16 == 0;
@@ -994,13 +999,14 @@ struct Builder {
         }
         // In one kernel where the convolution fits a pair tile, with the cheapest
         // length among a few times powers of two (planar data and uneven batches
-        // keep tile steps).  Convolutions of up to 64 points keep them too, but for a few
-        // rows: a tile of 32 rows goes through its element-wise passes row by row, which
-        // costs more than the saved intermediate (4 M points, us, one kernel / two
+        // keep tile steps).  Convolutions of up to 64 points keep them too where there are
+        // many rows: a tile of 32 rows goes through its element-wise passes row by row,
+        // which costs more than the saved intermediate (4 M points, us, one kernel / two
         // launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317; c2c 17 x 1 4.6 / 18,
-        // c2r 17 x 64 25 / 21).
+        // x 1927 21.5 / 23.4, c2r 17 x 64 25 / 21).
         PairChoice fused;
-        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= 16) && rows <= kPairMaxCols) {
+        const int64_t few = kind == 2 ? 16 : 16384;
+        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= few) && rows <= kPairMaxCols) {
             const int64_t pow2 = m;
             double best = 1e30;
             for (int64_t f : {1, 3, 5, 7, 9, 15}) {
@@ -1206,9 +1212,15 @@ struct Builder {
                 return add_multipass(n, outer, n, n, src, dst);
             // (even rows without a compile-time engine in two passes of pair tiles)
             if (n > 4096 && n <= kMaxSingleTileC2C && !p.use_tuned && p.precision == 0 && !tile_ends() &&
-                !find_static_kernel(static_cast<int>(n), IO_C2C) && long_row_in_two(n, outer)) {
-                p.pair_route = true;
-                return add_multipass(n, outer, n, n, src, dst);
+                !find_static_kernel(static_cast<int>(n), IO_C2C)) {
+                bool fits;
+                const bool two = long_row_in_two(n, outer, fits);
+                const bool both = fits && p.fft_type == 0x10 && p.sizes.size() == 1;
+                if (two || both) {
+                    p.pair_route = true;
+                    p.tile_first = !two;
+                    return add_multipass(n, outer, n, n, src, dst);
+                }
             }
             if (n <= std::min<int64_t>(kMaxSingleTileC2C, p.max_row_n) ||
                 (n <= std::min<int64_t>(kMaxRowN, p.max_row_n) && find_static_kernel(n, IO_C2C))) {
@@ -1576,7 +1588,8 @@ std::string describe_plan(const Plan &p)
         o << "\n";
     }
     if (!p.c32_base.empty()) {
-        o << "complex32 data: steps=" << p.c32_base.size() << "\n";
+        o << "complex32 data" << (p.tile_first ? ", and out of place from an aligned source" : "")
+          << ": steps=" << p.c32_base.size() << "\n";
         for (const Step &s : p.c32_base) o << "  " << s.what << "\n";
     }
     return o.str();

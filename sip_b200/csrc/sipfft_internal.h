@@ -288,6 +288,7 @@ struct Plan {
     // writes complex32 and separated data: routes that pay on the pair kernels are not taken.
     bool tile_ends = false;
     bool pair_route = false;  // (set by the planner) such a route was taken
+    bool tile_first = false;  // (and) it pays in place and from unaligned sources only: else c32_base runs
     // inverse STFT plan (asdFftIstftMakePlan): one column C2C step into workspace
     // slot 0 ([channel][frame][n_fft]), then the overlap-add kernel
     bool istft = false;
@@ -298,7 +299,7 @@ struct Plan {
     int precision = 0;
     // complex32 (FP16 pairs) variant of a 1D C2C plan's steps, built at the
     // first complex32 exec (c32_state: 0 not built, 1 built, -1 unsupported)
-    std::vector<Step> c32_base;  // the steps that it converts, where not `steps` (pair_route)
+    std::vector<Step> c32_base;  // the steps that it converts, where not `steps` (pair_route); of `tile_first`
     std::vector<Step> c32_steps;
     int c32_state = 0;
     bool forward() const;
