@@ -537,7 +537,10 @@ struct Builder {
             // A source that the row kernel's bulk copies cannot read stays on pair tiles (4 M points
             // at 8 bytes from alignment: c2c 3 points 34 us, 61).
             const bool few = d.io == IO_R2C_PACKED ? d.n < 6 || d.n == 8 : d.n < 14;
-            s.pair_unaligned = few && d.n_cols > 16384 && !p.use_tuned;
+            // Before another step the row kernel starts and ends apart (about 3 us more: 260 x 7 x 576 17
+            // on pair tiles, 20): from four times as many rows on.
+            const int64_t many = p.sizes.size() > 1 ? int64_t(1) << 18 : int64_t(1) << 16;
+            s.pair_unaligned = few && d.n_cols >= many && !p.use_tuned;
             // a tile of rows is copied as one run
             if (in_dist != d.n + (d.io == IO_C2R_PACKED ? 1 : 0)) return true;
         } else if (!p.use_tuned && d.n <= 32 && d.n_cols <= (d.n >= 9 ? 16 : 32) &&
@@ -631,8 +634,8 @@ struct Builder {
     // * with fewer than 16 columns, which fill no pass's tile (us, one-transform tiles / two passes /
     //   one: 500 x 7 x 1198 77 / 85 / 61, 729 x 7 x 6575 523 / 673 / 492, 768 x 7 x 48 16 / 17 / 16);
     // * for odd lengths below 900 with an odd number of columns, whose copies are 8 bytes either way,
-    //   while the data, its intermediate and the result fit L2 (r2c 729^2 x 7 71 / 78 / 68, 625^2 x 10
-    //   92 / 66 / 60; 945 x 65 x 68 84 / 65 / 72).
+    //   where the data, its intermediate and the result take half of L2 to all of it (r2c 729^2 x 7
+    //   71 / 78 / 68, 625^2 x 10 92 / 66 / 60; 945 x 65 x 68 84 / 65 / 72, 735^2 x 1 31 / 20 / 23).
     bool strided_axis_in_two(int64_t n, int64_t outer, int64_t inner) const
     {
         if (n <= 256 || n > kMaxStridedTile || inner <= 1) return false;
@@ -641,8 +644,9 @@ struct Builder {
         if (pair_columns(m) > 4) return false;
         if (n > 1024) return true;
         if (copies_bytes(n * inner, outer) / 3 > spare_copy_bytes(device)) return false;  // (no workspace)
+        const int64_t bytes = copies_bytes(n * inner, outer);
         const bool odd = n % 2 && inner % 2 && n < 900;
-        return inner >= 16 && !(odd && copies_bytes(n * inner, outer) <= kL2Bytes);
+        return inner >= 16 && !(odd && bytes > kL2Bytes / 2 && bytes <= kL2Bytes);
     }
 
     // the data of a step, its intermediate and the result
