@@ -634,7 +634,7 @@ struct Builder {
     // * with fewer than 16 columns, which fill no pass's tile (us, one-transform tiles / two passes /
     //   one: 500 x 7 x 1198 77 / 85 / 61, 729 x 7 x 6575 523 / 673 / 492, 768 x 7 x 48 16 / 17 / 16);
     // * for odd lengths below 900 with an odd number of columns, whose copies are 8 bytes either way,
-    //   where the data, its intermediate and the result take half of L2 to all of it (r2c 729^2 x 7
+    //   where the data, its intermediate and the result take a third of L2 to all of it (r2c 729^2 x 7
     //   71 / 78 / 68, 625^2 x 10 92 / 66 / 60; 945 x 65 x 68 84 / 65 / 72, 735^2 x 1 31 / 20 / 23).
     bool strided_axis_in_two(int64_t n, int64_t outer, int64_t inner) const
     {
@@ -646,7 +646,7 @@ struct Builder {
         if (copies_bytes(n * inner, outer) / 3 > spare_copy_bytes(device)) return false;  // (no workspace)
         const int64_t bytes = copies_bytes(n * inner, outer);
         const bool odd = n % 2 && inner % 2 && n < 900;
-        return inner >= 16 && !(odd && bytes > kL2Bytes / 2 && bytes <= kL2Bytes);
+        return inner >= 16 && !(odd && bytes > kL2Bytes / 3 && bytes <= kL2Bytes);
     }
 
     // the data of a step, its intermediate and the result
