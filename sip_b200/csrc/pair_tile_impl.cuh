@@ -580,9 +580,9 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_blue_kernel(const __grid
 // would need the whole grid resident, which other work on the GPU can prevent.)
 //
 // Everything an item needs is in shared memory before its turn: its ticket is
-// drawn four items ahead, its place in the list is copied (cp.async) three items
-// ahead, its descriptor two, its tile one (when its producer has finished;
-// otherwise at its turn).  (With all of that at its turn, a chain of four
+// drawn and its place in the list copied (cp.async) three items ahead, its
+// descriptor two, its tile one (when its producer has finished; otherwise at its
+// turn).  (With all of that at its turn, a chain of four
 // dependent global loads stood between two tiles: barrier and long-scoreboard
 // stalls were 5 of 12 cycles per instruction.)  The first tickets are drawn one
 // at a time, a load apart, so that short lists spread over the CTAs.
@@ -618,20 +618,22 @@ __global__ void __launch_bounds__(kPairThreads, 4)
     __shared__ __align__(8) int2 s_item[4];           // item k at [k & 3]
     __shared__ uint32_t s_known[kPairKnown / 32];     // producers seen finished
     __shared__ int s_flag;
+    // segment whose tile this CTA finished last, -1 if nobody waits for it.  (In shared memory,
+    // and no ticket held across a tile: the stages take every register, and the kernel's own that
+    // live across them spill.  76 bytes of spills cost 12 %: 20000 transforms 2.85 -> 2.51 ms.)
+    __shared__ int s_publish;
     const int tid = threadIdx.x;
-    uint32_t ticket = 0;  // thread 0: the list entry that this CTA takes next
-    auto draw = [&] {
-        if (tid == 0) ticket = atomicAdd(reinterpret_cast<unsigned *>(words + kBatchTicket), 1u);
+    if (tid == 0) s_publish = -1;
+    auto draw = [&]() -> uint32_t {
+        return tid == 0 ? atomicAdd(reinterpret_cast<unsigned *>(words + kBatchTicket), 1u) : 0u;
     };
-    draw();
     for (int i = tid; i < kPairKnown / 32; i += kPairThreads) s_known[i] = 0u;
-    auto place = [&](int k) {  // list entry of this CTA's item k, and the ticket of item k + 1
+    auto place = [&](int k, uint32_t ticket) {  // list entry of this CTA's item k
         if (tid != 0) return;
         if (ticket < static_cast<uint32_t>(nitems))
             cp_async8(&s_item[k & 3], items + ticket);
         else
             s_item[k & 3] = make_int2(-1, 0);
-        draw();
     };
     auto describe = [&](int k) {  // its descriptor (the entry has landed)
         const int sg = s_item[k & 3].x;
@@ -660,33 +662,31 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         const PairSeg &g = pair_slot(k % kPairSlots);
         pair_issue(g.d, source(g), pair_smem + kPairHeadWords + (k & 1) * buf_words, static_cast<uint32_t>(s_item[k & 3].y));
     };
-    place(0);
+    place(0, draw());
     cp_async_wait_all();
     __syncthreads();
     describe(0);
-    place(1);
+    place(1, draw());
     cp_async_wait_all();
     __syncthreads();
     // item 0 is the start of some segment's tiles: prefetched like the others
     bool staged = s_item[0].x >= 0 && ready(pair_slot(0), false);
     if (staged) copy_in(0);
     describe(1);
-    place(2);
-    int publish = -1;  // segment whose tile this CTA finished last
+    place(2, draw());
     for (int k = 0;; k++) {
+        // the ticket of item k + 3: its latency passes under the barrier and the copies' issue
+        const uint32_t ticket = draw();
         cp_async_wait_all();
         __syncthreads();  // item k's copies, k+1's descriptor and k+2's entry have landed; item k-1 is done
-        if (publish >= 0 && tid == 0) {
+        if (tid == 0 && s_publish >= 0) {
             __threadfence();
-            atomicAdd(words + kBatchDone + publish, 1);
+            atomicAdd(words + kBatchDone + s_publish, 1);
         }
         if (s_item[k & 3].x < 0) break;
         const PairSeg &g = pair_slot(k % kPairSlots);
         const bool more = s_item[(k + 1) & 3].x >= 0;
-        if (more) {
-            place(k + 3);
-            describe(k + 2);
-        }
+        if (more) describe(k + 2);
         if (!staged) {
             if (!ready(g, true)) break;  // the whole CTA: the results are incomplete, and reported as such
             copy_in(k);
@@ -695,9 +695,10 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         }
         staged = more && ready(pair_slot((k + 1) % kPairSlots), false);
         if (staged) copy_in(k + 1);
+        place(k + 3, ticket);
+        if (tid == 0) s_publish = g.consumed ? s_item[k & 3].x : -1;
         pair_tile<FWD, false>(k % kPairSlots, kPairHeadWords + (k & 1) * buf_words, source(g),
                               static_cast<char *>(bufs.p[g.out_buf]) + g.out_off, static_cast<uint32_t>(s_item[k & 3].y));
-        publish = g.consumed ? s_item[k & 3].x : -1;
     }
     cp_async_wait_all();
 }

@@ -8,7 +8,7 @@ import random
 
 import pytest
 
-AHEAD = 4  # tickets that a CTA holds beyond its current item
+AHEAD = 3  # tickets that a CTA holds beyond its current item
 
 
 def _work_list(rng):
