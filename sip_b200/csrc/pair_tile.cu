@@ -6,7 +6,7 @@
 
 namespace sipfft {
 
-// instantiated in pair_inst_fwd.cu and pair_inst_inv.cu
+// instantiated in pair_tile_fwd.cu / pair_tile_inv.cu and pair_batch_fwd.cu / pair_batch_inv.cu
 const void *pair_tile_fn_fwd();
 const void *pair_tile_fn_inv();
 const void *pair_batch_fn_fwd();

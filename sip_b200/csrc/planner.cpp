@@ -990,8 +990,10 @@ struct Builder {
 
     // Bluestein (chirp-z) N-point transform of contiguous rows for lengths
     // whose prime factors the codelets do not cover: a length-M circular
-    // convolution (M = 2^k >= 2N-1) done as two M-point FFT launches with the
-    // chirp pre/post multiplies and the precomputed FFT of the chirp fused in.
+    // convolution (M >= 2N-1) with the chirp pre/post multiplies and the
+    // precomputed FFT of the chirp fused in: one kernel (M up to 2048, a few times a
+    // power of two), two M-point FFT launches (M = 2^k up to 16384) or multi-pass
+    // FFTs with element-wise steps between them.
     // kind: 0 C2C, 1 R2C (real in, N/2+1 out), 2 C2R (N/2+1 in, real out).
     bool add_bluestein(int kind, int64_t n, int64_t rows, int64_t in_dist, int64_t out_dist, Buf src, Buf dst)
     {
