@@ -1011,8 +1011,9 @@ struct Builder {
         // launches: c2c 17 314 / 266, c2r 31 221 / 153; c2c 34 175 / 317; c2c 17 x 1 4.6 / 18,
         // x 1927 21.5 / 23.4, c2r 17 x 64 25 / 21).
         PairChoice fused;
-        const int64_t few = kind == 2 ? 16 : 16384;
-        if (p.fft_type != 0x30 && !p.use_tuned && (2 * n - 1 > 64 || rows <= few) && rows <= kPairMaxCols) {
+        const bool fuse = 2 * n - 1 > 64 || rows <= (kind == 2 ? 16 : 16384) ||
+                          rows * m > spare_copy_bytes(device) / int64_t(sizeof(float2));  // (no workspace)
+        if (p.fft_type != 0x30 && !p.use_tuned && fuse && rows <= kPairMaxCols) {
             const int64_t pow2 = m;
             double best = 1e30;
             for (int64_t f : {1, 3, 5, 7, 9, 15}) {

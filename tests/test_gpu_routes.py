@@ -189,6 +189,11 @@ def test_data_too_large_to_hold_once_more(cuda):
             assert st == fft.ACL_SUCCESS
             assert (fft.asdFftGetWorkspaceSize(h)[1] > 0) == fits, fft.describe_plan(h)
             fft.asdFftDestroy(h)
+    for rows, fits in ((quarter // (8 * 64), True), (quarter // (8 * 64) + 1, False)):  # 31 points by 64
+        h = fft.asdFftCreate()
+        assert fft.asdFftMakePlan1D(h, 31, C2C, FWD, rows) == fft.ACL_SUCCESS
+        assert (fft.asdFftGetWorkspaceSize(h)[1] > 0) == fits and ("in one kernel" in fft.describe_plan(h)) != fits
+        fft.asdFftDestroy(h)
     import ctypes
 
     lib = fft.load_library()
